@@ -28,6 +28,7 @@
 #include "../../include/ccpgpu.h"
 #include "analysis.h"
 #include "host.h"
+#include "fused.cuh"
 #include "kernels.cuh"
 #include "persist.cuh"
 
@@ -61,6 +62,11 @@ struct DevBuf {
 
 constexpr int TILE = 128;
 constexpr int SMALL_BATCH = 16384;  // beads: below, tiles of 64 and 8 lanes per bead
+// Batches up to this many beads step through k_fused (fused.cuh). us per step,
+// sorted path / k_fused: ccp 98304 beads 67.1 / 58.6 (more was not measured);
+// baseline 32768 beads 56.6 / 46.6, 65536 beads 73.0 / 85.0.
+constexpr int FUSED_MAX_WF = 100000, FUSED_MAX_LJ = 45000;
+constexpr int64_t FUSED_MAX_CELLS = 1 << 19;  // 1 KB a cell
 constexpr int MAX_CPS = 1024;  // cells per side of one system's grid
 constexpr uint32_t MAX_BATCH_BEADS = (1u << (32u - BF_BITS)) - 1u;
 constexpr int64_t MAX_BATCH_CELLS = (int64_t)INT32_MAX - 4 * (int64_t)SCAN_CHUNK;
@@ -169,6 +175,17 @@ struct Engine {
   int persist_reach = 0;
   size_t persist_bytes = 0;
   DevBuf<PGrid> d_pgrid;
+  // bucket path of small batches (fused.cuh), set up by its first steps
+  bool fused = false;
+  int fused_lanes = 8;                 // lanes per bead
+  int f_nc = 0, f_tiles = 0;           // bucket cells of all systems, CTAs
+  int fphase = 0;                      // count array (of three) that holds pos
+  bool buckets_valid = false;          // ... which is current
+  bool hist_valid = false;             // counts and rank are the histogram of pos
+  DevBuf<FusedGrid> d_fgrid;
+  DevBuf<Tile> d_ftiles;
+  DevBuf<float4> fslots[2], fovf[2];
+  DevBuf<uint32_t> fcnt;
 
   ~Engine() {
     for (auto &g : graphs) cudaGraphExecDestroy(g.second);
@@ -350,7 +367,145 @@ struct Engine {
     CK(cudaMemsetAsync(lbs_start.p, 0, sizeof(uint32_t) * (nc + 1), stream));
     reset_observables();
     setup_persist();
+    fused = !par.pair_path_given && persist_reach == 0 &&
+            nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) &&
+            fused_cells(nullptr) <= FUSED_MAX_CELLS;
     CK(cudaStreamSynchronize(stream));
+  }
+
+  // Bucket grids of all systems: cells of the largest pair cutoff, with a
+  // margin that keeps pairs at it within the stencil despite the rounding of
+  // the cell coordinates. Returns the number of cells.
+  int64_t fused_cells(std::vector<FusedGrid> *out) const {
+    const float csl = std::max(ff.rc_att, ff.rc_rep) * 1.0001f;
+    int64_t cells = 0;
+    for (size_t s = 0; s < hsys.size(); ++s) {
+      const float half = std::ceil(geo[s].d_m / csl);
+      if (!(half <= (float)(MAX_CPS / 2))) return FUSED_MAX_CELLS + 1;
+      const int64_t cps = std::max(2, 2 * (int)half) + 2;
+      if (out) out->push_back(FusedGrid{(int32_t)cells, (int32_t)cps, 1.0f / csl, 0});
+      cells += cps * cps * cps;
+      if (cells > FUSED_MAX_CELLS) return cells;
+    }
+    return cells;
+  }
+
+  // Sets the bucket path up on its first use; false: the batch steps through
+  // the sorted path (also when there is no memory left for the buckets).
+  bool setup_fused() {
+    if (!fused || d_fgrid.p) return fused;
+    std::vector<FusedGrid> g;
+    f_nc = (int)fused_cells(&g);
+    // More lanes per bead shorten a kernel until its CTAs (256 / lanes beads,
+    // three or four on an SM) no longer fit the GPU at once. us per step with
+    // 32 / 16 / 8 lanes, baseline: 2048 beads 12.2 / 16.2 / 26.2, 4096 beads
+    // 19.5 / 15.9 / 24.5, 8192 beads 28.7 / 25.6 / 25.1, 32768 beads - / 62.8 /
+    // 46.6; ccp: 2048 beads 9.0 / 9.5 / 13.3, 4096 beads 14.3 / 10.0 / 13.0,
+    // 8192 beads 20.4 / 15.7 / 13.9. Four lanes pay with ccp's small cells
+    // only: 32768 beads 26.3 (8) / 29.0 (4), 65536 beads 47.8 / 44.3.
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t fit = (int64_t)3 * sms * FUSED_PAIR_THREADS;
+    fused_lanes = (int64_t)nb * 32 <= fit ? 32 : ((int64_t)nb * 16 <= fit ? 16 : 8);
+    if (ff.pot == POT_WF && nb > 49152) fused_lanes = 4;
+    const int per = FUSED_PAIR_THREADS / fused_lanes;
+    std::vector<Tile> tl;
+    for (int s = 0; s < (int)hsys.size(); ++s)
+      for (int b = 0; b < hsys[s].n; b += per) tl.push_back(Tile{s, hsys[s].bead_off + b});
+    f_tiles = (int)tl.size();
+    try {
+      for (int k = 0; k < 2; ++k) {
+        fslots[k].alloc((size_t)f_nc * FUSED_CAP);
+        fovf[k].alloc(nb);
+      }
+      fcnt.alloc((size_t)3 * (f_nc + 1));
+      d_ftiles.alloc(tl.size());
+      d_fgrid.alloc(g.size());
+    } catch (const Error &) {
+      cudaGetLastError();
+      for (int k = 0; k < 2; ++k) {
+        fslots[k].release();
+        fovf[k].release();
+      }
+      fcnt.release();
+      d_ftiles.release();
+      return fused = false;
+    }
+    CK(cudaMemcpyAsync(d_ftiles.p, tl.data(), sizeof(Tile) * tl.size(), cudaMemcpyHostToDevice,
+                       stream));
+    CK(cudaMemcpyAsync(d_fgrid.p, g.data(), sizeof(FusedGrid) * g.size(), cudaMemcpyHostToDevice,
+                       stream));
+    CK(cudaStreamSynchronize(stream));
+    return true;
+  }
+
+  // Fills the buckets with the current positions.
+  void build_buckets() {
+    if (buckets_valid) return;
+    CK(cudaMemsetAsync(fcnt.p, 0, sizeof(uint32_t) * 3 * (f_nc + 1), stream));
+    k_fused_build<<<(unsigned)htiles.size(), tile, 0, stream>>>(
+        d_tiles.p, d_sys.p, d_fgrid.p, tile, pos.p, fcnt.p, fslots[0].p, fovf[0].p, f_nc, d_err.p);
+    CK(cudaGetLastError());
+    kcount += 1;
+    fphase = 0;
+    buckets_valid = true;
+  }
+
+  // One Heun stage; `phase`: the count array that holds its positions.
+  template <int STAGE>
+  void launch_fused(int phase, bool dependent) {
+    FusedArgs a;
+    a.tiles = d_ftiles.p;
+    a.sys = d_sys.p;
+    a.grid = d_fgrid.p;
+    a.pos = pos.p;
+    a.er = er.p;
+    a.fbuf = fbuf.p;
+    a.rnb = rnb.p;
+    a.slots_in = fslots[STAGE - 1].p;
+    a.slots_out = fslots[2 - STAGE].p;
+    a.ovf_in = fovf[STAGE - 1].p;
+    a.ovf_out = fovf[2 - STAGE].p;
+    const size_t stride = (size_t)f_nc + 1;
+    a.cnt_in = fcnt.p + stride * (phase % 3);
+    a.cnt_out = fcnt.p + stride * ((phase + 1) % 3);
+    a.cnt_zero = fcnt.p + stride * ((phase + 2) % 3);
+    a.lbs = lbs_sorted.p;
+    a.lbs_start = lbs_start.p;
+    a.step = d_step.p;
+    a.err = d_err.p;
+    a.n_cells = f_nc;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)f_tiles);
+    c.blockDim = dim3((unsigned)fused_threads(fused_lanes));
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = dependent ? 1 : 0;
+#define CCPGPU_FUSED(POT, S, G, MINB) CK(cudaLaunchKernelEx(&c, k_fused<STAGE, POT, S, G, MINB>, a, ff))
+    // S: cells hold 2-3 beads in ccp's field (side 2), 6 in the baseline (2.5)
+    if (ff.pot == POT_WF) {
+      if (fused_lanes == 32)
+        CCPGPU_FUSED(POT_WF, 4, 8, 3);
+      else if (fused_lanes == 16)
+        CCPGPU_FUSED(POT_WF, 4, 4, 3);
+      else if (fused_lanes == 8)
+        CCPGPU_FUSED(POT_WF, 4, 2, 4);
+      else
+        CCPGPU_FUSED(POT_WF, 4, 1, 3);
+    } else {
+      if (fused_lanes == 32)
+        CCPGPU_FUSED(POT_LJ, 8, 4, 3);
+      else if (fused_lanes == 16)
+        CCPGPU_FUSED(POT_LJ, 8, 2, 3);
+      else
+        CCPGPU_FUSED(POT_LJ, 8, 1, 4);
+    }
+#undef CCPGPU_FUSED
+    kcount += 1;
   }
 
   // Shared-memory cell grids of the persistent path: cells of the largest
@@ -483,6 +638,12 @@ struct Engine {
   }
 
   void recount() {
+    buckets_valid = false;  // the positions have changed
+    count_cells();
+  }
+
+  void count_cells() {
+    hist_valid = true;
     CK(cudaMemsetAsync(counts.p, 0, (size_t)nblk * SCAN_CHUNK, stream));
     k_count<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, counts.p,
                                                            rank.p, d_err.p);
@@ -783,7 +944,25 @@ struct Engine {
     launch_update<2, MODE>();
   }
 
+  // n Heun steps of the bucket path, two kernels each; the state at the first
+  // one is observed through the counting sort when obs is set.
+  void launch_fused_steps(int phase, int n, bool obs) {
+    if (obs) {
+      count_cells();
+      launch_scan(false);
+      launch_scatter(pos.p);
+      launch_observe_sorted(false);
+      hist_valid = false;
+    }
+    for (int k = 0; k < n; ++k) {
+      launch_fused<1>(phase + 2 * k, k > 0);
+      launch_fused<2>(phase + 2 * k + 1, true);
+    }
+  }
+
   // Graph of n steps; when obs is set the state at the first step is observed.
+  // mode: MODE_DST or MODE_ICG, or FUSED_KIND + phase for the bucket path.
+  static constexpr int FUSED_KIND = 16;
   cudaGraphExec_t graph_for(int mode, int n, bool obs) {
     auto key = std::make_tuple(mode, n, obs ? 1 : 0);
     auto it = graphs.find(key);
@@ -791,7 +970,8 @@ struct Engine {
     cudaGraph_t g;
     uint64_t k0 = kcount;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < n; ++k) {
+    if (mode >= FUSED_KIND) launch_fused_steps(mode - FUSED_KIND, n, obs);
+    for (int k = 0; k < n && mode < FUSED_KIND; ++k) {
       if (mode == MODE_DST)
         launch_step<MODE_DST>(obs && k == 0);
       else
@@ -884,6 +1064,8 @@ struct Engine {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     if (par.pair_kernel != 2 && par.pair_kernel != 4)
       throw Error(ST_ARG, "autotune needs a half-shell pair kernel");
+    const bool had_buckets = fused;
+    fused = false;
     download_positions();
     PinnedFloats saved_xyz = hxyz;
     uint64_t saved_step = step;
@@ -968,11 +1150,17 @@ struct Engine {
     }
     par.pair_lanes = best_lanes;
     regrid(csl, best_tile);
+    if (had_buckets) {  // the bucket path stays where it is faster than the best of these
+      fused = true;
+      const double ms = time_steps(reps);
+      fused = ms < best;
+      if (fused) best = ms;
+    }
     hxyz = saved_xyz;
     upload_positions();
     step = saved_step;
     rep << "], \"tile\": " << best_tile << ", \"lanes\": " << best_lanes
-        << ", \"tiles_tried\": [" << tt.str() << "], \"ms_per_step\": " << best << "}";
+        << ", \"buckets\": " << (fused ? 1 : 0) << ", \"tiles_tried\": [" << tt.str() << "], \"ms_per_step\": " << best << "}";
     return rep.str();
   }
 
@@ -984,6 +1172,8 @@ struct Engine {
     for (auto &x : e) CK(cudaEventCreate(&x));
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     set_device_step();
+    if (!hist_valid) count_cells();
+    buckets_valid = false;
     for (int r = 0; r < reps; ++r) {
       CK(cudaEventRecord(e[0], stream));
       launch_scan(true);
@@ -1043,7 +1233,18 @@ struct Engine {
       return;
     }
     set_device_step();
-    const int chunk = 128;
+    if (n == 0) return;
+    const bool buckets = mode == MODE_DST && setup_fused();
+    if (buckets) {
+      build_buckets();
+      hist_valid = false;
+    } else if (!hist_valid) {
+      count_cells();
+    }
+    buckets_valid = false;  // until every step is enqueued
+    // a multiple of 3: the bucket path's count arrays then start in the same
+    // phase and one graph serves every chunk
+    const int chunk = buckets ? 126 : 128;
     uint64_t left = n;
     while (left > 0) {
       int g;
@@ -1060,13 +1261,16 @@ struct Engine {
       } else {
         g = (int)std::min<uint64_t>(left, chunk);
       }
-      CK(cudaGraphLaunch(graph_for(mode, g, obs), stream));
-      kcount += graph_kernels[std::make_tuple(mode, g, obs ? 1 : 0)];
+      const int kind = buckets ? FUSED_KIND + fphase : mode;
+      CK(cudaGraphLaunch(graph_for(kind, g, obs), stream));
+      kcount += graph_kernels[std::make_tuple(kind, g, obs ? 1 : 0)];
+      if (buckets) fphase = (fphase + 2 * g) % 3;
       if (obs) ++frames_observed;
       step += g;
       dev_next += g;
       left -= g;
     }
+    buckets_valid = buckets;
   }
 
   // The persistent path: per chunk (a frame, at most 512 steps) the
@@ -1109,15 +1313,16 @@ struct Engine {
 
   // Standalone analysis at the current positions.
   void sort_now() {
+    if (!hist_valid) count_cells();
     launch_scan(false);
     launch_scatter(pos.p);
+    hist_valid = false;  // the scatter has used the histogram up
   }
 
   void observe(bool with_sdist) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     sort_now();
     launch_observe_sorted(with_sdist);
-    recount();
     CK(cudaGetLastError());
     ++frames_observed;
     sync_and_check();
@@ -1151,7 +1356,6 @@ struct Engine {
     k_observe<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, CCP_RCO / 2.0f, fobs.p);
     k_frame_extra<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, fextra.p);
     kcount += 2;
-    recount();
     CK(cudaGetLastError());
     ++frames_observed;
     std::vector<double> fo(ns * OBS_STRIDE), fx(ns * 2);
@@ -1239,7 +1443,6 @@ struct Engine {
     CK(cudaMemsetAsync(ovl.p, 0, sizeof(unsigned long long) * hsys.size(), stream));
     sort_now();
     launch_contacts_args(contact_args(false, false, true));
-    recount();
     CK(cudaGetLastError());
     std::vector<unsigned long long> o(hsys.size());
     CK(cudaMemcpyAsync(o.data(), ovl.p, sizeof(unsigned long long) * o.size(),
@@ -1254,7 +1457,6 @@ struct Engine {
     launch_pair<MODE_DST>();
     k_total_force<MODE_DST><<<(unsigned)htiles.size(), tile, 0, stream>>>(
         d_tiles.p, d_sys.p, ff, pos.p, fs.p, rank.p, lbs_sorted.p, lbs_start.p, fout.p);
-    recount();
     CK(cudaGetLastError());
     k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
     std::vector<float> f((size_t)3 * nb);

@@ -1,0 +1,369 @@
+// Heun stages of small batches in one kernel each.
+//
+// A batch that does not fill the GPU is bound by the launches of a step and
+// by the latency of each kernel, not by its arithmetic: scan (3), scatter,
+// pair and update, twice per step, are twelve kernels of 3-12 us each (12 to
+// 16 of 152 SMs busy at 2048 beads). Here a stage is one kernel, so a step is
+// two: positions live in fixed-capacity cell buckets, so no counting sort is
+// needed; every bead sums its own pair force over the full 27-cell stencil,
+// so no force is exchanged between beads; and the same CTA integrates its
+// beads and inserts their new positions into the next stage's buckets. The
+// full stencil costs two to three times the pair tests of the sorted half
+// stencil, which is what ends the range of this path.
+//
+// Measured on a GB300, us per Heun step, sorted path / this one (single
+// systems at ccp's chromatin volume fraction 0.125, baseline at packing
+// fraction 0.2):
+//   beads          1024         2048         8192         32768        98304
+//   ccp        38.4 /  8.6  39.8 /  9.0  41.7 / 13.6  47.9 / 26.3  68.3 / 58.6
+//   baseline   44.6 / 11.9  45.9 / 12.2  49.3 / 24.9  56.3 / 46.9  81.4 / 118
+//
+// Buckets. Every system has a grid of cells of side the largest pair cutoff.
+// A cell holds up to FUSED_CAP (x, y, z, index << 3 | flags) slots; beads
+// beyond that go to an overflow list that every bead scans (empty unless the
+// density is several times that of a relaxed system). There are two sets of
+// slots (positions and predictor) and three of counts: the kernel that reads
+// set k fills set k + 1 and clears set k + 2.
+//
+// CTA: 8 warps of pair lanes (L = S G lanes a bead, 256 / L beads), which also
+// take the lamina sites, and two threads a bead that meanwhile compute its
+// bonded and wall forces and its noise (one thread a bead for all of these,
+// sites included, took 12.9 instead of 9.5 us a step at 1024 ccp beads: its
+// serial chain was longer than the pair loop).
+#pragma once
+
+#include "kernels.cuh"
+
+namespace ccpgpu {
+
+constexpr int FUSED_CAP = 32;           // slots of a cell
+constexpr int FUSED_PAIR_THREADS = 256;
+// pair lanes, then a thread per bead for the other forces and one for the noise
+// (whole warps)
+__host__ __device__ constexpr int fused_own(int lanes) { return lanes > 8 ? 32 : FUSED_PAIR_THREADS / lanes; }
+__host__ __device__ constexpr int fused_threads(int lanes) { return FUSED_PAIR_THREADS + 2 * fused_own(lanes); }
+
+struct FusedGrid {  // one system's bucket grid, with a border of empty cells
+  int32_t cell_off, cps;  // cps: cells per side, border included
+  float inv_csl;
+  int32_t pad;
+};
+
+struct FusedArgs {
+  const Tile *tiles;  // 256 / L beads each
+  const SysDesc *sys;
+  const FusedGrid *grid;
+  float4 *pos, *er, *fbuf, *rnb;
+  const float4 *slots_in;
+  float4 *slots_out;
+  const uint32_t *cnt_in;  // per cell; [n_cells]: length of the overflow list
+  uint32_t *cnt_out, *cnt_zero;
+  const float4 *ovf_in;
+  float4 *ovf_out;
+  const float4 *lbs;
+  const uint32_t *lbs_start;
+  unsigned long long *step;
+  int *err;
+  int n_cells;
+};
+
+// Programmatic dependent launch: the next kernel's CTAs may start (and read
+// their constant tables) while this one runs; they wait here until every
+// write of the kernel before is visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ int fused_cell(float4 p, const FusedGrid &g, bool &esc) {
+  const int n = g.cps - 2;
+  const int x = cell_coord(p.x, g.inv_csl, n, esc), y = cell_coord(p.y, g.inv_csl, n, esc),
+            z = cell_coord(p.z, g.inv_csl, n, esc);
+  return g.cell_off + ((z + 1) * g.cps + y + 1) * g.cps + x + 1;
+}
+
+// Inserts bead i at p (flags in w) into its cell's bucket.
+__device__ __forceinline__ void fused_insert(float4 p, int i, const FusedGrid &g, uint32_t *cnt,
+                                             float4 *slots, float4 *ovf, int n_cells, int *err) {
+  bool esc = false;
+  const int c = fused_cell(p, g, esc);
+  if (esc) set_err(err, ERR_ESCAPE);
+  const float4 q = make_float4(p.x, p.y, p.z,
+                               __uint_as_float(((uint32_t)i << BF_BITS) | (wbits(p) & 7u)));
+  const uint32_t r = atomicAdd(&cnt[c], 1u);
+  if (r < (uint32_t)FUSED_CAP)
+    slots[(size_t)c * FUSED_CAP + r] = q;
+  else
+    ovf[atomicAdd(&cnt[n_cells], 1u)] = q;
+}
+
+// Buckets of the current positions (counts cleared by the host).
+__global__ void k_fused_build(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
+                              const FusedGrid *__restrict__ grid, int tile,
+                              const float4 *__restrict__ pos, uint32_t *cnt, float4 *slots,
+                              float4 *ovf, int n_cells, int *err) {
+  const Tile t = tiles[blockIdx.x];
+  const SysDesc &s = sys[t.sys];
+  const int i = t.begin + threadIdx.x;
+  if ((int)threadIdx.x >= tile || i >= s.bead_off + s.n) return;
+  fused_insert(pos[i], i, grid[t.sys], cnt, slots, ovf, n_cells, err);
+}
+
+// Whether the pair of the bead at p (word wi, `near` = (index - 1) << 3) and
+// the candidate q is within its class's cutoff and not |i - j| <= 1.
+__device__ __forceinline__ bool fused_hit(float4 p, uint32_t wi, uint32_t near, float4 q,
+                                          float rc2_att, float rc2_rep) {
+  const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+  const float d2 = dx * dx + dy * dy + dz * dz;
+  const uint32_t wj = wbits(q);
+  return d2 <= ((wi & wj & BF_HET) ? rc2_att : rc2_rep) && wj - near >= (3u << BF_BITS);
+}
+
+// Adds the pair's force on the bead at p; HH: both are A beads.
+template <int POT, bool HH>
+__device__ __forceinline__ void fused_add(float4 p, float4 q, const ForceField &ff, float3 &acc) {
+  const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+  const float d2 = dx * dx + dy * dy + dz * dz;
+  const float cf = POT == POT_WF ? wf_coef(ff.e_att, d2)
+                                 : lj_coef<!HH>(HH ? ff.e_att : ff.e_rep, dx, dy, dz, d2);
+  acc.x += cf * dx;
+  acc.y += cf * dy;
+  acc.z += cf * dz;
+}
+
+template <int POT>
+__device__ __forceinline__ void fused_test_add(float4 p, uint32_t wi, uint32_t near, float4 q,
+                                               float rc2_att, float rc2_rep, const ForceField &ff,
+                                               float3 &acc) {
+  if (!fused_hit(p, wi, near, q, rc2_att, rc2_rep)) return;
+  if (POT == POT_LJ && !(wi & wbits(q) & BF_HET))
+    fused_add<POT, false>(p, q, ff, acc);
+  else
+    fused_add<POT, true>(p, q, ff, acc);
+}
+
+// Offset of cell `it` (0 .. 26) of the stencil from its centre.
+__device__ __forceinline__ int fused_offset(int it, int cps) {
+  const int dz = it / 9, r = it - 9 * dz, dy = r / 3, dx = r - 3 * dy;
+  return ((dz - 1) * cps + dy - 1) * cps + dx - 1;
+}
+
+// Lamina-binding force on a LAD bead (lbs_force) from the (z, y) rows of cells
+// first, first + stride, ...: the bead's pair lanes take a row each.
+__device__ __forceinline__ float3 fused_lbs(float4 x, const SysDesc &s, const ForceField &ff,
+                                            const float4 *__restrict__ lbs,
+                                            const uint32_t *__restrict__ lbs_start, int first,
+                                            int stride) {
+  float3 f = make_float3(0.0f, 0.0f, 0.0f);
+  float d = sqrtf(x.x * x.x + x.y * x.y + x.z * x.z);
+  float m = ff.lco * 1.001f + 1e-4f;
+  if (d < s.lbs_rmin - m || d > s.lbs_rmax + m) return f;  // no site within reach
+  bool esc = false;
+  int xl = cell_coord(x.x - m, s.inv_csl, s.cps, esc), xh = cell_coord(x.x + m, s.inv_csl, s.cps, esc);
+  int yl = cell_coord(x.y - m, s.inv_csl, s.cps, esc), yh = cell_coord(x.y + m, s.inv_csl, s.cps, esc);
+  int zl = cell_coord(x.z - m, s.inv_csl, s.cps, esc), zh = cell_coord(x.z + m, s.inv_csl, s.cps, esc);
+  const float cl = ff.e_l * (8.0f / (3.0f * ff.lco * ff.lco));
+  const float l2h = __fmul_rn(ff.lco, ff.lco), l2l = __fmaf_rn(ff.lco, ff.lco, -l2h);
+  const int ny = yh - yl + 1, rows = ny * (zh - zl + 1);
+  for (int r = first; r < rows; r += stride) {
+    const int z = zl + r / ny, y = yl + r % ny;
+    int row = s.cell_off + (z * s.cps + y) * s.cps;
+    uint32_t b = lbs_start[row + xl], e = lbs_start[row + xh + 1];
+    for (uint32_t k = b; k < e; ++k) {
+      float4 q = lbs[k];
+      float vx = x.x - q.x, vy = x.y - q.y, vz = x.z - q.z;
+      // (d/lco)^6 - 1 = (n2 - 1)(n2^2 + n2 + 1) with n2 - 1 = (d^2 - lco^2) / lco^2:
+      // no cancellation as d -> lco, where the force goes to zero
+      float dd = sq3_minus(vx, vy, vz, l2h, l2l);
+      if (dd > 0.0f) continue;  // beyond the cutoff
+      float m1 = dd / l2h;
+      float n2 = 1.0f + m1;
+      float cf = cl * m1 * (n2 * n2 + n2 + 1.0f);
+      f.x += cf * vx;
+      f.y += cf * vy;
+      f.z += cf * vz;
+    }
+  }
+  return f;
+}
+
+// One Heun stage (see k_update): STAGE 1 reads pos and writes er, STAGE 2
+// reads er and writes pos. S lanes read the first S slots of a cell together
+// and G cells are read at once by the S G lanes of a bead. Every lane notes
+// its hits in a bit mask (one bit per cell visited) and evaluates them
+// afterwards: few candidates are within the cutoff, and evaluated in place
+// nearly every visit would run the coefficient for one or two lanes of 32.
+template <int STAGE, int POT, int S, int G, int MINB>
+__global__ void __launch_bounds__(fused_threads(S * G), MINB)
+    k_fused(const __grid_constant__ FusedArgs a, const __grid_constant__ ForceField ff) {
+  constexpr int L = S * G, B = FUSED_PAIR_THREADS / L;
+  constexpr int NV = (27 + G - 1) / G;
+  constexpr int OWN = fused_own(L), THREADS = fused_threads(L);
+  __shared__ float4 fpair[B], fnoise[B];
+  __shared__ int off[32];
+  const Tile t = a.tiles[blockIdx.x];
+  const SysDesc &s = a.sys[t.sys];
+  const FusedGrid g = a.grid[t.sys];
+  const int end = s.bead_off + s.n;
+  if (threadIdx.x < 32) off[threadIdx.x] = fused_offset(threadIdx.x, g.cps);
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  const float4 *X = (STAGE == 1) ? a.pos : a.er;
+  for (int c = blockIdx.x * THREADS + threadIdx.x; c <= a.n_cells;
+       c += gridDim.x * THREADS)
+    a.cnt_zero[c] = 0u;
+
+  float4 xi, r0, f1;
+  float3 F;
+  const int bo = (int)threadIdx.x - FUSED_PAIR_THREADS;  // bead of the own-force threads
+  const int io = t.begin + bo;
+  const bool mine = bo >= 0 && bo < B && io < end;
+  if (bo < 0) {
+    const int sub = threadIdx.x % L, b = threadIdx.x / L;
+    const int ss = sub % S, gs = sub / S;
+    const int i = t.begin + b;
+    const bool valid = i < end;
+    float3 acc = make_float3(0.0f, 0.0f, 0.0f);
+    const uint32_t n_ovf = a.cnt_in[a.n_cells];
+    const float4 p = X[valid ? i : t.begin];
+    const uint32_t wi = wbits(p), near = (uint32_t)(i - 1) << BF_BITS;
+    bool esc = false;
+    const int c0 = fused_cell(p, g, esc);
+    const float rc2_att = ff.rc_att * ff.rc_att, rc2_rep = ff.rc_rep * ff.rc_rep;
+    const uint32_t *cnt = a.cnt_in + c0;
+    const float4 *slots = a.slots_in + (size_t)c0 * FUSED_CAP + ss;
+    // one bit per cell visited: hits of A-A pairs, of other pairs, cells with
+    // more than S beads
+    uint32_t hit_a = 0, hit_x = 0, over = 0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int it = v * G + gs;
+      const int o = G == 1 ? fused_offset(v, g.cps) : off[it];
+      if (G == 1 || 27 % G == 0 || it < 27) {
+        // the slot is read without waiting for the count (a slot beyond it
+        // holds an old position and is not a hit)
+        const uint32_t n = cnt[o];
+        const float4 q = slots[(ptrdiff_t)o * FUSED_CAP];
+        if ((uint32_t)ss < n && fused_hit(p, wi, near, q, rc2_att, rc2_rep)) {
+          if (POT == POT_LJ && !(wi & wbits(q) & BF_HET))
+            hit_x |= 1u << v;
+          else
+            hit_a |= 1u << v;
+        }
+        if (n > (uint32_t)S) over |= 1u << v;
+      }
+    }
+    if (!valid) hit_a = hit_x = over = 0;
+    while (__any_sync(0xffffffffu, hit_a != 0u)) {
+      if (hit_a) {
+        const int o = off[(__ffs(hit_a) - 1) * G + gs];
+        hit_a &= hit_a - 1u;
+        fused_add<POT, true>(p, slots[(ptrdiff_t)o * FUSED_CAP], ff, acc);
+      }
+    }
+    if (POT == POT_LJ) {
+      while (__any_sync(0xffffffffu, hit_x != 0u)) {
+        if (hit_x) {
+          const int o = off[(__ffs(hit_x) - 1) * G + gs];
+          hit_x &= hit_x - 1u;
+          fused_add<POT, false>(p, slots[(ptrdiff_t)o * FUSED_CAP], ff, acc);
+        }
+      }
+    }
+    while (over) {  // cells with more than S beads
+      const int o = off[(__ffs(over) - 1) * G + gs];
+      over &= over - 1u;
+      const uint32_t n = min(cnt[o], (uint32_t)FUSED_CAP);
+      for (uint32_t k = S + ss; k < n; k += S)
+        fused_test_add<POT>(p, wi, near, slots[(ptrdiff_t)o * FUSED_CAP + (k - ss)], rc2_att, rc2_rep,
+                            ff, acc);
+    }
+    if (n_ovf && valid) {
+      for (uint32_t k = sub; k < n_ovf; k += L) {
+        const float4 q = a.ovf_in[k];
+        const int gj = (int)(wbits(q) >> BF_BITS);
+        if (gj >= s.bead_off && gj < end)
+          fused_test_add<POT>(p, wi, near, q, rc2_att, rc2_rep, ff, acc);
+      }
+    }
+    if ((wi & BF_LAD) && valid && s.n_lbs > 0) {
+      const float3 fl3 = fused_lbs(p, s, ff, a.lbs, a.lbs_start, sub, L);
+      acc.x += fl3.x;
+      acc.y += fl3.y;
+      acc.z += fl3.z;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+      acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+    }
+    if (sub == 0) fpair[b] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+  } else if (bo >= OWN) {
+    // the noise warp: stage 1 draws, stage 2 takes what stage 1 drew
+    const int in = io - OWN;
+    if (bo - OWN < B && in < end) {
+      float3 z = make_float3(0.0f, 0.0f, 0.0f);
+      if (ff.sd > 0.0f) {
+        if (STAGE == 1) {
+          // the counter holds the last step taken; the second stage advances it
+          z = bead_noise((uint32_t)(in - s.bead_off), *a.step + 1ull, s.seed_lo, s.seed_hi, a.err);
+          z = make_float3(ff.sd * z.x, ff.sd * z.y, ff.sd * z.z);
+          a.rnb[in] = make_float4(z.x, z.y, z.z, 0.0f);
+        } else {
+          const float4 r4 = a.rnb[in];
+          z = make_float3(r4.x, r4.y, r4.z);
+        }
+      }
+      fnoise[bo - OWN] = make_float4(z.x, z.y, z.z, 0.0f);
+    }
+  } else if (mine) {
+    // the neighbours are read at once: their flags decide what is used
+    xi = X[io];
+    float4 nb[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      nb[k] = X[min(max(io + (k < 2 ? k - 2 : k - 1), s.bead_off), end - 1)];
+    if (STAGE == 2) {
+      r0 = a.pos[io];
+      f1 = a.fbuf[io];
+    }
+    F = bonded_force_at([&](int j) { return j < io ? nb[j - io + 2] : nb[j - io + 1]; }, io, xi, end,
+                        ff);
+    float3 vw;
+    float gh, gl;
+    if (wall_vector<MODE_DST>(make_float3(xi.x, xi.y, xi.z), s, vw, gh, gl)) {
+      const float cw = wall_coef<MODE_DST>(gh, gl, ff);
+      F.x += cw * vw.x;
+      F.y += cw * vw.y;
+      F.z += cw * vw.z;
+    }
+  }
+  __syncthreads();
+  if (!mine) return;
+  const float4 fp = fpair[bo], rn = fnoise[bo];
+  F.x += fp.x;
+  F.y += fp.y;
+  F.z += fp.z;
+  float4 out;
+  if (STAGE == 1) {
+    float3 D = make_float3(F.x * ff.dt, F.y * ff.dt, F.z * ff.dt);
+    cap_step(D, ff.max_step);
+    out = make_float4(xi.x + D.x + rn.x, xi.y + D.y + rn.y, xi.z + D.z + rn.z, xi.w);
+    a.er[io] = out;
+    a.fbuf[io] = make_float4(F.x, F.y, F.z, 0.0f);
+  } else {
+    const float h = 0.5f * ff.dt;
+    float3 D = make_float3((f1.x + F.x) * h, (f1.y + F.y) * h, (f1.z + F.z) * h);
+    cap_step(D, ff.max_step);
+    out = make_float4(r0.x + D.x + rn.x, r0.y + D.y + rn.y, r0.z + D.z + rn.z, r0.w);
+    a.pos[io] = out;
+    if (blockIdx.x == 0 && bo == 0) *a.step += 1ull;
+  }
+  if (!(isfinite(out.x) && isfinite(out.y) && isfinite(out.z))) set_err(a.err, ERR_NAN);
+  fused_insert(out, io, g, a.cnt_out, a.slots_out, a.ovf_out, a.n_cells, a.err);
+}
+
+}  // namespace ccpgpu

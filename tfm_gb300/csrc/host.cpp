@@ -227,6 +227,7 @@ Params parse_params(const std::string &text) {
   if (!(p.pair_lanes == 0 || p.pair_lanes == 1 || p.pair_lanes == 2 || p.pair_lanes == 4 ||
         p.pair_lanes == 8))
     fail("pair_lanes out of range");
+  p.pair_path_given = pm.has("pair_kernel") || pm.has("pair_lanes") || pm.has("cell_side");
   p.persistent = pm.get<int>("persistent", 0);
   if (!(p.persistent == 0 || p.persistent == 1)) fail("persistent out of range");
   if (!(p.n_chains >= 1 && (uint32_t)p.n_chains <= p.N)) fail("number_of_chains out of range");

@@ -79,6 +79,8 @@ struct Params {
   // 1: when every system fits one CTA's shared memory, steps run in the
   // persistent per-system kernel (one launch per frame); 0: graph path
   int persistent = 0;
+  // the text chooses the pair kernel, its lanes or the cell side
+  bool pair_path_given = false;
   std::string sequence_file = "Program/data/sequence.txt";
   ForceField ff{};
 };
