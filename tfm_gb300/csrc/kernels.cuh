@@ -1692,10 +1692,38 @@ __device__ __forceinline__ bool walk_in_cone(const WalkChain &w, double la, doub
 // accepted lane is the attempt the sequential walk accepts; a chunk never
 // extends past the attempt that triggers a move back. So the walk equals the
 // sequential one. Chunks start at one attempt and double after each chunk
-// that is rejected whole (up to 32), so a walk that is mostly accepted keeps
-// one lane busy. wxyz holds the FP64 positions the walk continues from; pos
+// that is rejected whole (up to 32).
+// The walk is bound by the FP64 pipe, which a warp instruction holds for
+// about 64 cycles however few of its lanes are active. So what depends on the
+// draw alone (~160 of the ~200 FP64 instructions of an attempt: sincospi,
+// log1p, erfinv) is computed for 32 draws at once, one a lane; a single
+// attempt's vector operations are spread over three lanes; and the wall test
+// compares squares. wxyz holds the FP64 positions the walk continues from; pos
 // receives them in FP32. A chain that exceeds its draw budget sets ERR_WALK.
-constexpr int WALK_WARPS = 4;
+constexpr int WALK_WARPS = 1;
+
+struct WalkDraw {
+  double3 dir;        // random direction
+  double cb, sn, lb;  // cosine and sine of the bond angle, bond length
+};
+
+__device__ __forceinline__ WalkDraw walk_draw(const WalkChain &w, const WalkParams &wp, uint32_t d) {
+  const U32x4 r = walk_bits(w, d);
+  WalkDraw o;
+  o.dir = walk_direction(r.x, r.y);
+  // cos of the bond angle by inversion of its density exp(c_b cos) on [-1, 1]
+  double cb = 1.0 + log1p(-wp.one_m_e * walk_u(r.z)) * wp.inv_cb;
+  if (cb > 1.0) cb = 1.0;  // comparisons keep a NaN (rejected, like acos(NaN))
+  if (cb < -1.0) cb = -1.0;
+  o.cb = cb;
+  o.sn = sqrt(1.0 - cb * cb);
+  o.lb = wp.l_0 + wp.sig_b * erfinv(2.0 * walk_u(r.w) - 1.0);
+  return o;
+}
+
+__device__ __forceinline__ double walk_pick(double3 v, int c) {
+  return c == 0 ? v.x : (c == 1 ? v.y : v.z);
+}
 
 __global__ void __launch_bounds__(32 * WALK_WARPS)
 k_random_walk(const WalkChain *__restrict__ chains, int n_chains, WalkParams wp,
@@ -1753,48 +1781,83 @@ k_random_walk(const WalkChain *__restrict__ chains, int n_chains, WalkParams wp,
   int att = 0;
   int i = w.first + 1;
   chunk = 1;
+  // lane l holds what draw base + l gives whatever the walk's state: a random
+  // direction, the bond angle's cosine and sine and the bond length
+  uint32_t base = draw;
+  WalkDraw wd = walk_draw(w, wp, base + lane);
+  const double d2_in = r_in * r_in * (1.0 - 1e-12), d2_out = r_in * r_in * (1.0 + 1e-12);
+  const int cn = lane == 2 ? 0 : lane + 1, cp = lane == 0 ? 2 : lane - 1;  // lanes of components
   while (i < w.end) {
-    const int m = (att >= 1024) ? 1 : min(chunk, 1025 - att);
+    if (draw - base == 32u) {
+      base = draw;
+      wd = walk_draw(w, wp, base + lane);
+    }
+    const int at = (int)(draw - base);
+    const int m = min((att >= 1024) ? 1 : min(chunk, 1025 - att), 32 - at);
     if (draw + (uint32_t)m > w.max_draws) {
       if (lane == 0) set_err(err, ERR_WALK);
       break;
     }
-    double3 p = prev, nd = old;
+    double3 p, nd;
     bool ok = false;
-    if (lane < m) {
-      U32x4 r = walk_bits(w, draw + lane);
-      double3 rd = walk_direction(r.x, r.y);
-      double3 per = make_double3(old.y * rd.z - old.z * rd.y, old.z * rd.x - old.x * rd.z,
-                                 old.x * rd.y - old.y * rd.x);
-      double il = rsqrt(per.x * per.x + per.y * per.y + per.z * per.z);
-      // cos of the bond angle by inversion of its density exp(c_b cos) on [-1, 1]
-      double cb = 1.0 + log1p(-wp.one_m_e * walk_u(r.z)) * wp.inv_cb;
-      if (cb > 1.0) cb = 1.0;  // comparisons keep a NaN (rejected, like acos(NaN))
-      if (cb < -1.0) cb = -1.0;
-      double sb = sqrt(1.0 - cb * cb) * il;
+    const int from = m == 1 ? at : min(at + lane, 31);
+    const double3 rd = make_double3(__shfl_sync(FULL, wd.dir.x, from), __shfl_sync(FULL, wd.dir.y, from),
+                                    __shfl_sync(FULL, wd.dir.z, from));
+    const double cb = __shfl_sync(FULL, wd.cb, from), sn = __shfl_sync(FULL, wd.sn, from),
+                 lb = __shfl_sync(FULL, wd.lb, from);
+    if (m == 1) {
+      // one attempt: lanes 0-2 compute a component each (every FP64
+      // instruction occupies the pipe for a whole warp)
+      const double o1 = walk_pick(old, cn), o2 = walk_pick(old, cp);
+      const double r1 = walk_pick(rd, cn), r2 = walk_pick(rd, cp);
+      const double per = o1 * r2 - o2 * r1;
+      const double px = __shfl_sync(FULL, per, 0), py = __shfl_sync(FULL, per, 1),
+                   pz = __shfl_sync(FULL, per, 2);
+      const double sb = sn * rsqrt(px * px + py * py + pz * pz);
+      const double n = cb * walk_pick(old, lane) + sb * per;
+      const double q = lb * n + walk_pick(prev, lane);
+      nd = make_double3(__shfl_sync(FULL, n, 0), __shfl_sync(FULL, n, 1), __shfl_sync(FULL, n, 2));
+      p = make_double3(__shfl_sync(FULL, q, 0), __shfl_sync(FULL, q, 1), __shfl_sync(FULL, q, 2));
+    } else {
+      const double3 per = make_double3(old.y * rd.z - old.z * rd.y, old.z * rd.x - old.x * rd.z,
+                                       old.x * rd.y - old.y * rd.x);
+      const double sb = sn * rsqrt(per.x * per.x + per.y * per.y + per.z * per.z);
       nd = make_double3(cb * old.x + sb * per.x, cb * old.y + sb * per.y, cb * old.z + sb * per.z);
-      double lb = wp.l_0 + wp.sig_b * erfinv(2.0 * walk_u(r.w) - 1.0);
       p = make_double3(lb * nd.x + prev.x, lb * nd.y + prev.y, lb * nd.z + prev.z);
-      double dr = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
-      ok = isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && !((w.R_n - dr) < wp.mis) &&
-           walk_in_cone(w, la, p, dr);
+    }
+    if (lane < m) {
+      const double d2 = p.x * p.x + p.y * p.y + p.z * p.z;
+      // the wall test R - d < mis needs the root only at its very edge
+      bool far = d2 < d2_in;
+      double dr = 0.0;
+      if (!far && !(d2 > d2_out)) {
+        dr = sqrt(d2);
+        far = !((w.R_n - dr) < wp.mis);
+      }
+      ok = far && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+      if (ok && la != 0.0) ok = walk_in_cone(w, la, p, sqrt(d2));
     }
     unsigned acc = __ballot_sync(FULL, ok);
     // the accepted candidate, or the last rejected one, stays stored at bead i
     const int j = acc ? __ffs(acc) - 1 : m - 1;
     if (lane == j) {
-      float4 v = pos[i];
-      pos[i] = make_float4((float)p.x, (float)p.y, (float)p.z, v.w);
+      float4 v = make_float4((float)p.x, (float)p.y, (float)p.z, pos[i].w);
+      pos[i] = v;
       double *q = wxyz + 3 * (size_t)i;
       q[0] = p.x;
       q[1] = p.y;
       q[2] = p.z;
     }
     if (acc) {
-      old = make_double3(__shfl_sync(FULL, nd.x, j), __shfl_sync(FULL, nd.y, j),
-                         __shfl_sync(FULL, nd.z, j));
-      prev = make_double3(__shfl_sync(FULL, p.x, j), __shfl_sync(FULL, p.y, j),
-                          __shfl_sync(FULL, p.z, j));
+      if (m == 1) {
+        old = nd;
+        prev = p;
+      } else {
+        old = make_double3(__shfl_sync(FULL, nd.x, j), __shfl_sync(FULL, nd.y, j),
+                           __shfl_sync(FULL, nd.z, j));
+        prev = make_double3(__shfl_sync(FULL, p.x, j), __shfl_sync(FULL, p.y, j),
+                            __shfl_sync(FULL, p.z, j));
+      }
       draw += (uint32_t)j + 1u;
       att = 0;
       chunk = 1;
