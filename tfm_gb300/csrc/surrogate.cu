@@ -133,6 +133,8 @@ static const DevInfo &dev_info() {
     SCK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     SCK(cudaDeviceGetAttribute(&d.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     SCK(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
+    SCK(cudaFuncSetAttribute(k_conv_rows<ROWS_FORWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
+    SCK(cudaFuncSetAttribute(k_conv_rows<ROWS_GRADIENT>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
     dev_seen = dev;
   }
   return d;
@@ -177,6 +179,10 @@ struct Launcher {
         throw Error(ST_ARG, "tap pattern not supported (3x3, 1x5, 1x3 or 1x1 grids)");
     if (std::abs(sh.step_w) * (C / 2) > WIN_RADIUS) throw Error(ST_ARG, "tap column offset above the window radius");
     const int cb = cin / 64;
+    if (R == 3 && cb == 1 && N == 64 && sh.step_h != 0) {
+      conv_rows(x, w, B, H, W, sh.step_h, sh.step_w, epi);
+      return;
+    }
     sh.stages = MAX_STAGES;
     while (sh.stages > MMA_WARPS && (int)conv_smem_bytes(nt, cb, N, sh.stages) > d.max_smem)
       sh.stages -= MMA_WARPS;
@@ -198,11 +204,47 @@ struct Launcher {
     launched = true;                                                                           \
   }
 #define SUR_CONV_N(R_, C_, CB_) SUR_CONV(64, R_, C_, CB_) SUR_CONV(128, R_, C_, CB_)
+    // (64, 3, 3, 1): rows that all read the same input row; the rest is conv_rows
     SUR_CONV_N(3, 3, 1) SUR_CONV_N(3, 3, 2) SUR_CONV_N(1, 5, 1) SUR_CONV_N(1, 5, 2)
     SUR_CONV_N(1, 3, 1) SUR_CONV_N(1, 3, 2) SUR_CONV_N(1, 1, 1) SUR_CONV_N(1, 1, 2)
 #undef SUR_CONV_N
 #undef SUR_CONV
     if (!launched) throw Error(ST_ARG, "convolution configuration not instantiated");
+    SCK(cudaGetLastError());
+    ++kernels;
+  }
+
+  // The 3x3, 64 -> 64 channel case of conv, every input row read once. The
+  // next kernel's CTAs start as this one's leave their SMs and load their
+  // weights before its end.
+  void conv_rows(const CUtensorMap &x, const CUtensorMap &w, int B, int H, int W, int step_h, int step_w,
+                 const ConvEpi &epi) {
+    const DevInfo &d = dev_info();
+    RowsShape sh{};
+    sh.H = H;
+    sh.W = W;
+    sh.d = std::abs(step_h);
+    sh.sgn = step_h > 0 ? 1 : -1;
+    sh.step_w = step_w;
+    sh.total = B * (W / 128) * H;
+    if (sh.total == 0) return;
+    const int kind = epi.out_f32 ? ROWS_GRADIENT : ROWS_FORWARD, grid = std::min(sh.total, d.sms);
+    const uint32_t smem = rows_smem_bytes(kind);
+    if ((int)smem > d.max_smem) throw Error(ST_ARG, "convolution weights do not fit in shared memory");
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3(ROWS_THREADS);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    if (kind == ROWS_GRADIENT)
+      SCK(cudaLaunchKernelEx(&c, k_conv_rows<ROWS_GRADIENT>, x, w, sh, epi, err));
+    else
+      SCK(cudaLaunchKernelEx(&c, k_conv_rows<ROWS_FORWARD>, x, w, sh, epi, err));
     SCK(cudaGetLastError());
     ++kernels;
   }
@@ -635,6 +677,7 @@ struct Net {
       e.bias = params.p + ly.b_off;
       e.relu = 1;
       e.resid = z[l].p;
+      e.resid_is_input = 1;
       // the last layer's output is needed only by the backward pass
       e.out = (!last || training) ? z[l + 1].p : nullptr;
       e.mask_out = training ? hmask[l + 1].p : nullptr;

@@ -87,6 +87,7 @@ struct ConvEpi {
   const float *wo, *bo;     // [64], [1]
   float *y;                 // [P]
   const float *resid_dy;    // [P]: adds resid_dy[p] * wo[c] (the output layer's gradient)
+  int resid_is_input;       // resid is the convolution's input image (k_conv_rows)
 };
 
 // shared memory after the operand tiles: barriers (256 B), TMEM slot and
@@ -469,6 +470,447 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   if (warp == 1) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, TMEM_COLS_CONV);
+  }
+  if (threadIdx.x == 0 && *abort) atomicOr(err, 1);
+}
+
+// ------------------------------------------------------------------ 3x3 convolution, 64 channels
+
+// The head's 3x3 convolution (64 -> 64 channels) with every input row read
+// once. A CTA walks down runs of output rows that are step_h apart; the window
+// of one input row is multiplied by the three taps of a column at once
+// (N = 192: the weights of tap rows 2, 1, 0 one after the other) into the
+// accumulators of the three output rows it belongs to, which lie side by side
+// in TMEM. Against one output row at a time (k_conv_tc, N = 64) the tensor
+// core reads 4 KB of pixels and 6 KB of weights for three taps instead of
+// 3 x (4 + 2) KB: a 128 x 64 x 16 MMA is bound by these reads (48 cycles), a
+// 128 x 192 x 16 one by the multipliers (96); and a window is copied from L2
+// once instead of three times.
+//
+// An output row receives its tap rows in the order 0, 1, 2, each column by
+// column, as in k_conv_tc, so the FP32 sums have the same bits.
+//
+// Measured on a GB300, 128 maps of 256^2, a forward layer, us: k_conv_tc 640;
+// this kernel with one issuing lane inside a divergent branch 485, with the
+// issue loop run by the converged warp 400. What bounds it now: HBM (2.2 GB read
+// and written: 330 us at the measured copy rate) with the MMAs (250 us) close
+// behind. Running six layers over groups of images small enough for L2 was
+// slower (8.7 instead of 7.7 ms for 300 maps at 8 images a group): a launch
+// costs 5 us to fill and drain the pipeline.
+constexpr int ROWS_SLOTS = 8;       // accumulators of 64 TMEM columns
+constexpr int ROWS_GROUPS = 2;      // groups of EPI_WARPS, taking alternate output rows
+constexpr int ROWS_THREADS = 32 * (2 + ROWS_GROUPS * EPI_WARPS);
+constexpr uint32_t ROWS_W_BYTES = 9u * 64u * 128u;
+
+// Which fields of the epilogue apply. ROWS_FORWARD: bias, relu, mask_out,
+// resid, out and the output layer; ROWS_GRADIENT: resid_f32, resid_dy, out_f32,
+// mask_in, out.
+enum : int { ROWS_FORWARD = 0, ROWS_GRADIENT = 1 };
+
+// input windows in shared memory, and the staging tile of an epilogue warp's
+// 32 pixels x 32 channels (BF16 or FP32)
+__host__ __device__ constexpr int rows_stages(int kind) { return kind == ROWS_FORWARD ? 6 : 4; }
+__host__ __device__ constexpr uint32_t rows_stage_bytes(int kind) {
+  return kind == ROWS_FORWARD ? 2048u : 4096u;
+}
+__host__ __device__ constexpr uint32_t rows_smem_bytes(int kind) {
+  return 1024u + ROWS_W_BYTES + (uint32_t)rows_stages(kind) * WIN_BYTES + CONV_SMEM_TAIL +
+         (uint32_t)(ROWS_GROUPS * EPI_WARPS) * rows_stage_bytes(kind);
+}
+
+struct RowsShape {
+  int H, W;    // W: a multiple of 128
+  int d, sgn;  // tap rows read input row h + (r - 1) sgn d
+  int step_w;
+  int total;  // output rows of 128 pixels: images * (W / 128) * H
+};
+
+// A run of output rows: row q (0 .. n - 1) is image row h0 + sgn d q of the
+// 128-pixel column block wb of image b.
+struct RowRun {
+  int b, wb, h0, n;
+};
+
+// The run at flat row f (column block by column block, in a block the rows
+// h = 0, d, 2d, ... then 1, 1 + d, ...), at most to f1; f moves behind it.
+__device__ __forceinline__ bool rows_next(const RowsShape &sh, int &f, int f1, RowRun &r) {
+  if (f >= f1) return false;
+  const int col = f / sh.H, wt = sh.W >> 7;
+  int g = f - col * sh.H, c = 0, nc;
+  for (;; ++c) {
+    nc = (sh.H - c + sh.d - 1) / sh.d;
+    if (g < nc) break;
+    g -= nc;
+  }
+  r.b = col / wt;
+  r.wb = col - r.b * wt;
+  r.n = min(nc - g, f1 - f);
+  r.h0 = sh.sgn > 0 ? c + g * sh.d : c + (nc - 1 - g) * sh.d;
+  f += r.n;
+  return true;
+}
+
+// 32 FP32 channels of 32 pixels, one pixel a lane, to or from global memory
+// through the warp's staging tile: an instruction moves 4 pixels' contiguous
+// 128 bytes (16-byte chunks XOR-swizzled by pixel against bank conflicts).
+__device__ __forceinline__ void rows_load_f32(const float *src, size_t pbase, int c0, float4 *r) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    r[i] = reinterpret_cast<const float4 *>(src + (pbase + (size_t)(4 * i + (lane >> 3))) * 64 +
+                                            c0)[lane & 7];
+}
+
+__device__ __forceinline__ void rows_add_f32(const float4 *r, float *v, float4 *stage) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int pr = 4 * i + (lane >> 3);
+    stage[pr * 8 + ((lane & 7) ^ (pr & 7))] = r[i];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float4 q = stage[lane * 8 + (k ^ (lane & 7))];
+    v[4 * k] += q.x;
+    v[4 * k + 1] += q.y;
+    v[4 * k + 2] += q.z;
+    v[4 * k + 3] += q.w;
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void rows_store_f32(float *dst, size_t pbase, int c0, const float *v,
+                                               float4 *stage) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    stage[lane * 8 + (k ^ (lane & 7))] =
+        make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int pr = 4 * i + (lane >> 3);
+    reinterpret_cast<float4 *>(dst + (pbase + (size_t)pr) * 64 + c0)[lane & 7] =
+        stage[pr * 8 + ((lane & 7) ^ (pr & 7))];
+  }
+  __syncwarp();
+}
+
+// tmx: 4-D map over the input {64, W, H, B} with box {64, WIN_ROWS, 1, 1};
+// tmw: 2-D map over the weights {64, 9 x 64} with box {64, 64}; 128-byte
+// swizzle. Grid: at most one CTA per SM; each takes an equal share of the rows.
+// Warp 0: TMA, warp 1: MMA issue, warps 2-17: epilogue, two groups of eight that
+// take alternate rows (one group's serial chain of an accumulator load, the
+// arithmetic and the stores took 2600 cycles a row, the MMAs 1200). In
+// ROWS_FORWARD they also hold on to the windows: a residual that is the
+// convolution's own input is read there.
+template <int KIND>
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
+    k_conv_rows(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
+                const RowsShape sh, const ConvEpi e, int *err) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = tc::smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  constexpr int S = rows_stages(KIND);
+  const uint32_t w_base = base;
+  const uint32_t a_base = w_base + ROWS_W_BYTES;
+  const uint32_t bar0 = a_base + (uint32_t)S * WIN_BYTES;
+  // barriers: full[S], empty[S], tfull[8], tempty[8], weights, fin
+  const uint32_t full0 = bar0, empty0 = bar0 + 8u * S, tfull0 = bar0 + 16u * S,
+                 tempty0 = tfull0 + 8u * ROWS_SLOTS, wbar = tempty0 + 8u * ROWS_SLOTS, fin = wbar + 8u;
+  uint8_t *tail = smem_raw + (bar0 + 256u - raw);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tail);
+  volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  float *sbias = reinterpret_cast<float *>(tail + 256);
+  float *swo = sbias + 128;
+  uint4 *epi_stage = reinterpret_cast<uint4 *>(smem_raw + (bar0 + CONV_SMEM_TAIL - raw));
+
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      tc::mbar_init(full0 + 8u * s, 1);
+      tc::mbar_init(empty0 + 8u * s, KIND == ROWS_FORWARD ? 1 + EPI_WARPS : 1);
+    }
+    for (int b = 0; b < ROWS_SLOTS; ++b) {
+      tc::mbar_init(tfull0 + 8u * b, 1);
+      tc::mbar_init(tempty0 + 8u * b, EPI_WARPS);
+    }
+    tc::mbar_init(wbar, 1);
+    tc::mbar_init(fin, 1);
+    *abort = 0;
+    tc::fence_barrier_init();
+  }
+  if (threadIdx.x < 64) {
+    sbias[threadIdx.x] = e.bias ? e.bias[threadIdx.x] : 0.0f;
+    swo[threadIdx.x] = e.wo ? e.wo[threadIdx.x] : 0.0f;
+  }
+  if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), 64u * ROWS_SLOTS);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  int f = (int)((long long)sh.total * blockIdx.x / gridDim.x);
+  const int f1 = (int)((long long)sh.total * (blockIdx.x + 1) / gridDim.x);
+  RowRun run;
+  tc::pdl_trigger();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tc::prefetch_map(&tmx);
+      tc::prefetch_map(&tmw);
+      // tap (r, c) goes to tile 3 c + 2 - r: the taps of a column side by side
+      tc::mbar_arrive_expect_tx(wbar, ROWS_W_BYTES);
+      for (int r = 0; r < 3; ++r)
+        for (int c = 0; c < 3; ++c)
+          tc::tma_load_2d(w_base + (uint32_t)(3 * c + 2 - r) * 8192u, &tmw, wbar, 0, (3 * r + c) * 64);
+      tc::pdl_wait();  // the weights are older than the kernel before
+      uint32_t n = 0;  // windows issued
+      bool ok = true;
+      while (ok && rows_next(sh, f, f1, run)) {
+        for (int j = 0; j < run.n + 2; ++j, ++n) {
+          const uint32_t slot = n % (uint32_t)S;
+          if (!tc::mbar_wait(empty0 + 8u * slot, ((n / (uint32_t)S) & 1u) ^ 1u, abort)) {
+            ok = false;
+            break;
+          }
+          tc::mbar_arrive_expect_tx(full0 + 8u * slot, WIN_BYTES);
+          tc::tma_load_4d(a_base + slot * WIN_BYTES, &tmx, full0 + 8u * slot, 0,
+                          run.wb * 128 - WIN_RADIUS, run.h0 + (j - 1) * sh.sgn * sh.d, run.b);
+        }
+      }
+      // nothing may still be landing in shared memory when the CTA exits
+      tc::mbar_drain(wbar, 0);
+      for (uint32_t k = n - min(n, (uint32_t)S); k < n; ++k)
+        tc::mbar_drain(full0 + 8u * (k % (uint32_t)S), (k / (uint32_t)S) & 1u);
+    }
+  } else if (warp == 1) {
+    // the whole warp runs the loop, so that the descriptors stay in uniform
+    // registers; lane 0 issues
+    const uint32_t mine = lane == 0 ? 1u : 0u;
+    {
+      constexpr uint32_t id64 = tc::idesc_bf16(128, 64, false, false);
+      const uint64_t desc_hi = tc::sdesc(0u, 16u, 1024u);
+      const uint32_t col_step = (uint32_t)(sh.step_w * 128);
+      uint32_t s = 0, ph = 0;  // window slot and phase
+      uint32_t q0 = 0;         // output rows of the runs before
+      bool ok = tc::mbar_wait(wbar, 0, abort);
+      while (ok && rows_next(sh, f, f1, run)) {
+        const int n = run.n;
+        for (int j = 0; j < n + 2; ++j) {
+          // input row j belongs to output rows j - 2 .. j
+          const int lo = max(0, j - 2), n_old = min(n - 1, j - 1) - lo + 1;
+          const bool fresh = j < n;
+          const uint32_t qn = q0 + (uint32_t)j;
+          if (fresh &&
+              !tc::mbar_wait(tempty0 + 8u * (qn % ROWS_SLOTS), ((qn / ROWS_SLOTS) & 1u) ^ 1u, abort)) {
+            ok = false;
+            break;
+          }
+          if (!tc::mbar_wait(full0 + 8u * s, ph, abort)) {
+            ok = false;
+            break;
+          }
+          tc::fence_after_sync();
+          const uint32_t a0 = a_base + s * WIN_BYTES + WIN_RADIUS * 128u - col_step;
+          // accumulators [lo .. j] in TMEM; those that wrap around its end
+          // take a second instruction
+          const uint32_t slot = (q0 + (uint32_t)lo) % ROWS_SLOTS;
+          const uint32_t cnt = (uint32_t)n_old + (fresh ? 1u : 0u);
+          const uint32_t n1 = min(cnt, (uint32_t)ROWS_SLOTS - slot), n2 = cnt - n1;
+          const uint32_t b0 = w_base + (uint32_t)(lo - (j - 2)) * 8192u;
+          const uint32_t d1 = tmem + slot * 64u;
+          // N = 64 x accumulators: the descriptor's N field counts units of 8
+          const uint32_t id1 = id64 + ((n1 - 1u) << 20), id2 = id64 + ((n2 - 1u) << 20);
+          // the first instruction of the new row starts its accumulator
+          const uint32_t o1 = min((uint32_t)n_old, (uint32_t)ROWS_SLOTS - slot), o2 = (uint32_t)n_old - o1;
+          const uint64_t ad = desc_hi | (a0 >> 4), bd = desc_hi | (b0 >> 4);
+          if (o1) tc::mma_bf16_warp(mine, d1, ad, bd, id64 + ((o1 - 1u) << 20), 1u);
+          if (o2) tc::mma_bf16_warp(mine, tmem, ad, bd + o1 * 512u, id64 + ((o2 - 1u) << 20), 1u);
+          if (fresh)
+            tc::mma_bf16_warp(mine, tmem + (qn % ROWS_SLOTS) * 64u, ad, bd + (uint32_t)n_old * 512u, id64, 0u);
+          if (n2 == 0u) {
+#pragma unroll
+            for (int t = 1; t < 12; ++t) {
+              const int c = t >> 2, k = t & 3;
+              tc::mma_bf16_warp(mine, d1, desc_hi | ((a0 + (uint32_t)c * col_step + 32u * k) >> 4),
+                           bd + (uint32_t)(c * 1536 + 2 * k), id1, 1u);
+            }
+          } else {
+#pragma unroll
+            for (int t = 1; t < 12; ++t) {
+              const int c = t >> 2, k = t & 3;
+              const uint64_t a = desc_hi | ((a0 + (uint32_t)c * col_step + 32u * k) >> 4);
+              const uint64_t b = bd + (uint32_t)(c * 1536 + 2 * k);
+              tc::mma_bf16_warp(mine, d1, a, b, id1, 1u);
+              tc::mma_bf16_warp(mine, tmem, a, b + n1 * 512u, id2, 1u);
+            }
+          }
+          tc::mma_commit_warp(mine, empty0 + 8u * s);
+          if (j >= 2) tc::mma_commit_warp(mine, tfull0 + 8u * ((qn - 2u) % ROWS_SLOTS));
+          if (++s == (uint32_t)S) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        q0 += (uint32_t)n;
+      }
+      tc::mma_commit_warp(mine, fin);
+      tc::mbar_drain(fin, 0);
+    }
+  } else {
+    // ---- epilogue: warp w reads TMEM lanes 32 (w mod 4) .. +31, half of the columns
+    const int qd = warp & 3, half = ((warp - 2) >> 2) & 1, group = (warp - 2) >> 3;
+    const int c0 = 32 * half, row = qd * 32 + lane;
+    uint4 *stage = epi_stage + (warp - 2) * (rows_stage_bytes(KIND) / 16);
+    uint32_t q = 0;  // output rows
+    uint32_t w = 0;  // windows
+    // Every window is released by one group (and by the MMAs that read it),
+    // after it has been filled: an arrival before that would count for the
+    // slot's previous window. A group waits for windows at most six apart
+    // (the MMAs of its row before have read all up to five behind), so the
+    // parity names the right phase.
+    auto window_wait = [&](uint32_t n) {
+      return tc::mbar_wait(full0 + 8u * (n % (uint32_t)S), (n / (uint32_t)S) & 1u, abort);
+    };
+    // The fence orders a lane's reads before the copy that the arrival allows:
+    // without it (and with the loads' values not yet used) the arrival overtook
+    // them, and one pass in fifteen returned wrong pixels.
+    auto window_done = [&](uint32_t n) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(empty0 + 8u * (n % (uint32_t)S));
+    };
+    bool ok = true;
+    tc::pdl_wait();
+    while (ok && rows_next(sh, f, f1, run)) {
+      for (int k = 0; k < run.n; ++k, ++q) {
+        if ((int)(q % ROWS_GROUPS) != group) continue;
+        const size_t pb = ((size_t)run.b * sh.H + (run.h0 + k * sh.sgn * sh.d)) * sh.W +
+                          (size_t)run.wb * 128 + qd * 32;
+        const size_t p = pb + lane;
+        const uint32_t slot = q % ROWS_SLOTS, own = w + (uint32_t)k + 1u;  // own row's window
+        if (KIND == ROWS_FORWARD && k == 0) {  // the halo row above the run
+          if (!window_wait(w)) {
+            ok = false;
+            break;
+          }
+          window_done(w);
+        }
+        // global inputs, before the accumulator is ready
+        uint4 rb[4];
+        float4 rf[8];
+        uint32_t mi = 0;
+        float rdy = 0.0f;
+        if (KIND == ROWS_FORWARD) {
+          if (e.resid && !e.resid_is_input) load_row_bf16x32<64>(e.resid, pb, c0, rb, stage);
+        } else {
+          if (e.resid_f32) rows_load_f32(e.resid_f32, pb, c0, rf);
+          if (e.mask_in) mi = e.mask_in[p * 2 + half];
+          if (e.resid_dy) rdy = e.resid_dy[p];
+        }
+        if ((KIND == ROWS_FORWARD && !window_wait(own)) ||
+            !tc::mbar_wait(tfull0 + 8u * slot, (q / ROWS_SLOTS) & 1u, abort)) {
+          ok = false;
+          break;
+        }
+        if (KIND == ROWS_FORWARD) {
+          if (e.resid_is_input) {
+            // this row's own pixels lie in the window it was computed from
+            const uint4 *win =
+                reinterpret_cast<const uint4 *>(smem_raw + (a_base + (own % (uint32_t)S) * WIN_BYTES - raw)) +
+                (WIN_RADIUS + row) * 8;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) rb[t] = win[(4 * half + t) ^ ((WIN_RADIUS + row) & 7)];
+          }
+        }
+        tc::fence_after_sync();
+        float v[32];
+        tc::tmem_ld32(tmem + ((uint32_t)(qd * 32) << 16) + slot * 64u + (uint32_t)c0, v);
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(tempty0 + 8u * slot);
+        const float4 *w4 = reinterpret_cast<const float4 *>(swo + c0);
+        if (KIND == ROWS_FORWARD) {
+          const float4 *b4 = reinterpret_cast<const float4 *>(sbias + c0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 b = b4[i];
+            v[4 * i] += b.x;
+            v[4 * i + 1] += b.y;
+            v[4 * i + 2] += b.z;
+            v[4 * i + 3] += b.w;
+          }
+          if (e.mask_out) {
+            uint32_t bits = 0;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) bits |= (v[i] > 0.0f ? 1u : 0u) << i;
+            e.mask_out[p * 2 + half] = bits;
+          }
+          if (e.relu) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.0f);
+          }
+          if (e.resid) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t r[4] = {rb[i].x, rb[i].y, rb[i].z, rb[i].w};
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                v[8 * i + 2 * t] += bf_lo(r[t]);
+                v[8 * i + 2 * t + 1] += bf_hi(r[t]);
+              }
+            }
+          }
+          window_done(own);
+          if (e.y) {
+            float dot = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 o = w4[i];
+              dot = fmaf(o.x, __bfloat162float(__float2bfloat16_rn(v[4 * i])), dot);
+              dot = fmaf(o.y, __bfloat162float(__float2bfloat16_rn(v[4 * i + 1])), dot);
+              dot = fmaf(o.z, __bfloat162float(__float2bfloat16_rn(v[4 * i + 2])), dot);
+              dot = fmaf(o.w, __bfloat162float(__float2bfloat16_rn(v[4 * i + 3])), dot);
+            }
+            // two terms onto the zeroed y: their order does not matter
+            atomicAdd(e.y + p, half == 0 ? dot + e.bo[0] : dot);
+          }
+        } else {
+          if (e.resid_f32) rows_add_f32(rf, v, reinterpret_cast<float4 *>(stage));
+          if (e.resid_dy) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 o = w4[i];
+              v[4 * i] = fmaf(rdy, o.x, v[4 * i]);
+              v[4 * i + 1] = fmaf(rdy, o.y, v[4 * i + 1]);
+              v[4 * i + 2] = fmaf(rdy, o.z, v[4 * i + 2]);
+              v[4 * i + 3] = fmaf(rdy, o.w, v[4 * i + 3]);
+            }
+          }
+          if (e.out_f32) rows_store_f32(e.out_f32, pb, c0, v, reinterpret_cast<float4 *>(stage));
+          if (e.mask_in) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = ((mi >> i) & 1u) ? v[i] : 0.0f;
+          }
+        }
+        if (e.out) store_row_bf16x32<64>(e.out, pb, c0, v, stage);
+        if (KIND == ROWS_FORWARD && k == run.n - 1) {  // the halo row below it
+          if (!window_wait(own + 1u)) {
+            ok = false;
+            break;
+          }
+          window_done(own + 1u);
+        }
+      }
+      w += (uint32_t)run.n + 2u;
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 64u * ROWS_SLOTS);
   }
   if (threadIdx.x == 0 && *abort) atomicOr(err, 1);
 }

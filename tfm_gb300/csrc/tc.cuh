@@ -37,6 +37,14 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
+// Programmatic dependent launch: a kernel launched as a dependent may start
+// while the one before still runs; pdl_wait returns when that one is complete
+// and its writes are visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------------------ mbarrier
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -207,6 +215,28 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// mma_bf16 for a converged warp: executed by the lane whose `mine` is not 0
+// (one lane, the same for all of a pipeline's MMAs and commits).
+__device__ __forceinline__ void mma_bf16_warp(uint32_t mine, uint32_t d_tmem, uint64_t adesc,
+                                              uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(mine)
+      : "memory");
+}
+
+__device__ __forceinline__ void mma_commit_warp(uint32_t mine, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+      "r"(mine)
       : "memory");
 }
 
