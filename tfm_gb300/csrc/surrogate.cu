@@ -133,6 +133,7 @@ static const DevInfo &dev_info() {
     SCK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     SCK(cudaDeviceGetAttribute(&d.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     SCK(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
+    SCK(cudaFuncSetAttribute(k_wgrad_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
     SCK(cudaFuncSetAttribute(k_conv_rows<ROWS_FORWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
     SCK(cudaFuncSetAttribute(k_conv_rows<ROWS_GRADIENT>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));
     dev_seen = dev;
@@ -281,16 +282,55 @@ struct Launcher {
     chunks = (sh.kb_total + sh.kb_per_cta - 1) / sh.kb_per_cta;
   }
 
-  static size_t partial_floats(int B, int H, int W, int cin, int N, int ntaps, bool want_db) {
+  // Taps of a 3x3 grid whose rows are step_h and columns step_w apart.
+  static bool grid3(const Taps &taps, int &step_h, int &step_w) {
+    if (taps.size() != 9) return false;
+    step_h = taps[8].first;
+    step_w = taps[8].second;
+    for (int t = 0; t < 9; ++t)
+      if (taps[t].first != (t / 3 - 1) * step_h || taps[t].second != (t % 3 - 1) * step_w) return false;
+    return true;
+  }
+
+  // Whether k_wgrad_rows computes these gradients: 64 -> 64 channels, images
+  // of whole 128-pixel blocks, and the window's margin covers the taps.
+  static bool wgrad_by_rows(int W, int cin, int N, const Taps &taps, int &step_h, int &step_w) {
+    return cin == 64 && N == 64 && W % 128 == 0 && grid3(taps, step_h, step_w) && step_h != 0 && step_w > 0 &&
+           step_w <= WIN_RADIUS;
+  }
+
+  static size_t partial_floats(int B, int H, int W, int cin, int N, const Taps &taps, bool want_db) {
+    int step_h, step_w;
+    if (wgrad_by_rows(W, cin, N, taps, step_h, step_w))
+      return (size_t)std::min(B * H, dev_info().sms) * WR_ATOMS * 4096;
     WgradShape sh;
     int chunks, groups;
     uint32_t smem;
-    plan_wgrad(B, H, W, cin, N, ntaps, want_db, sh, chunks, groups, smem);
+    plan_wgrad(B, H, W, cin, N, (int)taps.size(), want_db, sh, chunks, groups, smem);
     return (size_t)chunks * sh.n_atoms * N * 64;
   }
 
-  void wgrad(const CUtensorMap &x64, const CUtensorMap &y64, int B, int H, int W, int cin, int N, const Taps &taps,
-             float *partial, size_t partial_cap, float *dw, float *db) {
+  // x64, y64: maps with boxes of 64 pixels, x128: of WIN_ROWS pixels.
+  void wgrad(const CUtensorMap &x64, const CUtensorMap &x128, const CUtensorMap &y64, int B, int H, int W, int cin,
+             int N, const Taps &taps, float *partial, size_t partial_cap, float *dw, float *db) {
+    RowsShape rs{};
+    int step_h = 0;
+    if (wgrad_by_rows(W, cin, N, taps, step_h, rs.step_w)) {
+      rs.H = H;
+      rs.W = W;
+      rs.d = std::abs(step_h);
+      rs.sgn = step_h > 0 ? 1 : -1;
+      rs.total = B * H;
+      if (rs.total == 0) return;
+      const int grid = std::min(rs.total, dev_info().sms);
+      if ((size_t)grid * WR_ATOMS * 4096 > partial_cap) throw Error(ST_STATE, "partial-sum buffer too small");
+      k_wgrad_rows<<<grid, WG_THREADS, wgrad_rows_smem_bytes(), st>>>(x128, y64, rs, partial, err);
+      SCK(cudaGetLastError());
+      k_wgrad_reduce<<<9 * 64 + (db ? 64 : 0), 256, 0, st>>>(partial, grid, WR_ATOMS, 9, 64, 1, dw, db);
+      SCK(cudaGetLastError());
+      kernels += 2;
+      return;
+    }
     WgradShape sh;
     int chunks, groups;
     uint32_t smem;
@@ -631,10 +671,9 @@ struct Net {
     m_duv_128 = image_map(duv.p, 128, M, 1, B, WIN_ROWS);
     dhp.alloc(PM * 128);
     size_t pc = 0;
-    pc = std::max(pc, Launcher::partial_floats(B, M, M, 64, 64, 9, true));
-    pc = std::max(pc, Launcher::partial_floats(B, 1, M, 128, 128, 1, true));
-    pc = std::max(pc, Launcher::partial_floats(B, 1, L, 128, 128, cfg.enc_kernel, true));
-    pc = std::max(pc, Launcher::partial_floats(B, 1, L, 64, 128, cfg.enc_kernel, true));
+    for (const Layer &ly : head) pc = std::max(pc, Launcher::partial_floats(B, M, M, 64, 64, ly.off, true));
+    pc = std::max(pc, Launcher::partial_floats(B, 1, M, 128, 128, proj.off, true));
+    for (const Layer &ly : enc) pc = std::max(pc, Launcher::partial_floats(B, 1, L, ly.cin, 128, ly.off, true));
     partial.alloc(pc);
   }
 
@@ -705,7 +744,7 @@ struct Net {
     int kz = -1;  // dz_{l+1} is in hdz[kz]; -1: the rank-1 dy wo of the output layer
     for (int l = HL - 1; l >= 0; --l) {
       const Layer &ly = head[l];
-      run.wgrad(m_z_64[l], m_hdc_64[kc], n, M, M, 64, 64, ly.off, partial.p, partial.n, grads.p + ly.w_off,
+      run.wgrad(m_z_64[l], m_z_128[l], m_hdc_64[kc], n, M, M, 64, 64, ly.off, partial.p, partial.n, grads.p + ly.w_off,
                 grads.p + ly.b_off);
       ConvEpi e{};
       if (kz >= 0) {
@@ -730,7 +769,7 @@ struct Net {
     k_dist_reduce<<<blocks((long long)M * 64), 256, 0, st>>>(dist_part.p, M, n, grads.p + E_off);
     SCK(cudaGetLastError());
     run.kernels += 3;
-    run.wgrad(m_hp_64, m_duv_64, n, 1, M, 128, 128, proj.off, partial.p, partial.n, grads.p + proj.w_off,
+    run.wgrad(m_hp_64, m_hp_128, m_duv_64, n, 1, M, 128, 128, proj.off, partial.p, partial.n, grads.p + proj.w_off,
               grads.p + proj.b_off);
     {
       ConvEpi e{};
@@ -744,7 +783,7 @@ struct Net {
     int ke = 0;
     for (int l = EL - 1; l >= 1; --l) {
       const Layer &ly = enc[l];
-      run.wgrad(m_h_64[l], m_edc_64[ke], n, 1, L, 128, 128, ly.off, partial.p, partial.n, grads.p + ly.w_off,
+      run.wgrad(m_h_64[l], m_h_128[l], m_edc_64[ke], n, 1, L, 128, 128, ly.off, partial.p, partial.n, grads.p + ly.w_off,
                 grads.p + ly.b_off);
       ConvEpi e{};
       e.resid_f32 = edz[ke].p;
@@ -754,7 +793,7 @@ struct Net {
       run.conv(m_edc_128[ke], ly.map_wt, n, 1, L, 128, 128, negated(ly.off), e);
       ke ^= 1;
     }
-    run.wgrad(m_x0_64, m_edc_64[ke], n, 1, L, 64, 128, enc[0].off, partial.p, partial.n, grads.p + enc[0].w_off,
+    run.wgrad(m_x0_64, m_x0_128, m_edc_64[ke], n, 1, L, 64, 128, enc[0].off, partial.p, partial.n, grads.p + enc[0].w_off,
               grads.p + enc[0].b_off);
   }
 
@@ -1199,7 +1238,7 @@ int ccpsur_wgrad_bf16(int32_t B, int32_t H, int32_t W, int32_t cin, int32_t cout
     if (db_out) dbo.alloc(cout);
     derr.alloc(1);
     derr.zero(st);
-    part.alloc(Launcher::partial_floats(B, H, W, cin, cout, ntaps, db_out != nullptr));
+    part.alloc(Launcher::partial_floats(B, H, W, cin, cout, taps, db_out != nullptr));
     SCK(cudaMemcpyAsync(dx.p, x, P * cin * 2, cudaMemcpyHostToDevice, st));
     SCK(cudaMemcpyAsync(ddy.p, dy, P * cout * 2, cudaMemcpyHostToDevice, st));
     Launcher run;
@@ -1207,7 +1246,7 @@ int ccpsur_wgrad_bf16(int32_t B, int32_t H, int32_t W, int32_t cin, int32_t cout
     run.err = derr.p;
     CUtensorMap mx = image_map(dx.p, cin, W, H, B, 64);
     CUtensorMap my = image_map(ddy.p, cout, W, H, B, 64);
-    run.wgrad(mx, my, B, H, W, cin, cout, taps, part.p, part.n, dwo.p, db_out ? dbo.p : nullptr);
+    run.wgrad(mx, image_map(dx.p, cin, W, H, B, WIN_ROWS), my, B, H, W, cin, cout, taps, part.p, part.n, dwo.p, db_out ? dbo.p : nullptr);
     int flags = 0;
     SCK(cudaMemcpyAsync(dw_out, dwo.p, (size_t)ntaps * cout * cin * 4, cudaMemcpyDeviceToHost, st));
     if (db_out) SCK(cudaMemcpyAsync(db_out, dbo.p, cout * 4, cudaMemcpyDeviceToHost, st));

@@ -522,7 +522,8 @@ struct RowsShape {
   int H, W;    // W: a multiple of 128
   int d, sgn;  // tap rows read input row h + (r - 1) sgn d
   int step_w;
-  int total;  // output rows of 128 pixels: images * (W / 128) * H
+  int total;  // rows shared out: of 128 pixels (k_conv_rows: images * (W / 128) * H)
+              // or whole (k_wgrad_rows: images * H)
 };
 
 // A run of output rows: row q (0 .. n - 1) is image row h0 + sgn d q of the
@@ -531,22 +532,51 @@ struct RowRun {
   int b, wb, h0, n;
 };
 
-// The run at flat row f (column block by column block, in a block the rows
-// h = 0, d, 2d, ... then 1, 1 + d, ...), at most to f1; f moves behind it.
+// Rows h = c, c + d, ... of one image or column block are its class c; position
+// g counts the rows class by class. The class of position g (made the position
+// within the class), and the class's number of rows.
+__device__ __forceinline__ int rows_class(const RowsShape &sh, int &g, int &nc) {
+  int c = 0;
+  for (;; ++c) {
+    nc = (sh.H - c + sh.d - 1) / sh.d;
+    if (g < nc) return c;
+    g -= nc;
+  }
+}
+
+__device__ __forceinline__ int rows_begin(const RowsShape &sh, int c, int g, int nc) {
+  return sh.sgn > 0 ? c + g * sh.d : c + (nc - 1 - g) * sh.d;
+}
+
+// The run at flat row f (column block by column block), at most to f1; f moves
+// behind it.
 __device__ __forceinline__ bool rows_next(const RowsShape &sh, int &f, int f1, RowRun &r) {
   if (f >= f1) return false;
   const int col = f / sh.H, wt = sh.W >> 7;
-  int g = f - col * sh.H, c = 0, nc;
-  for (;; ++c) {
-    nc = (sh.H - c + sh.d - 1) / sh.d;
-    if (g < nc) break;
-    g -= nc;
-  }
+  int g = f - col * sh.H, nc;
+  const int c = rows_class(sh, g, nc);
   r.b = col / wt;
   r.wb = col - r.b * wt;
   r.n = min(nc - g, f1 - f);
-  r.h0 = sh.sgn > 0 ? c + g * sh.d : c + (nc - 1 - g) * sh.d;
+  r.h0 = rows_begin(sh, c, g, nc);
   f += r.n;
+  return true;
+}
+
+// The same for whole image rows f .. f1 (image by image): the run of the next
+// column block wb, f moving on after the last one.
+__device__ __forceinline__ bool bands_next(const RowsShape &sh, int &f, int &wb, int f1, RowRun &r) {
+  if (f >= f1) return false;
+  r.b = f / sh.H;
+  int g = f - r.b * sh.H, nc;
+  const int c = rows_class(sh, g, nc);
+  r.wb = wb;
+  r.n = min(nc - g, f1 - f);
+  r.h0 = rows_begin(sh, c, g, nc);
+  if (++wb == (sh.W >> 7)) {
+    wb = 0;
+    f += r.n;
+  }
   return true;
 }
 
@@ -1068,6 +1098,208 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   if (warp == 1) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, (uint32_t)sh.tmem_cols);
+  }
+  if (threadIdx.x == 0 && *abort) atomicOr(err, 2);
+}
+
+// Weight and bias gradients of the 3x3, 64 -> 64 channel convolution with every
+// input row and every gradient row read once (k_wgrad_tc copies the input once a
+// tap: 80 KB from L2 for 64 pixels, which bounds it). A CTA walks down the runs
+// of a band of whole image rows, as many pixels as k_wgrad_tc gives a CTA: the
+// tensor core's FP32 sums round towards zero, so their error grows with their
+// length, and it stays what it was. One input row's window meets the gradient
+// rows q = j - 2, j - 1, j it belongs to (tap rows 2, 1, 0) as one N = 192
+// operand, 128 pixels deep; two column shifts of the window stack into M = 128,
+// the third column and an all-ones block (the bias) into a second. Accumulators:
+// 2 x 192 TMEM columns, tap row r in columns 64 (2 - r) of each.
+//
+// Measured on a GB300, 32 maps of 256^2, us a layer: k_wgrad_tc 237, this
+// kernel 130; HBM floor 80 (537 MB), MMAs 83 (16 of 96 cycles a row of 128 pixels).
+constexpr int WR_X = 4, WR_Y = 6;           // windows and gradient rows in shared memory
+constexpr uint32_t WR_Y_BYTES = 128u * 128u;
+constexpr int WR_ATOMS = 10;                // nine taps, all-ones
+
+__host__ __device__ constexpr uint32_t wgrad_rows_smem_bytes() {
+  return 1024u + WR_X * WIN_BYTES + (WR_Y + 1) * WR_Y_BYTES + 256u;
+}
+
+// partial[blockIdx.x][tap or ones][co][ci]. tmx: map over X {64, W, H, B} with
+// box {64, WIN_ROWS, 1, 1}, tmy: map over dY with box {64, 64, 1, 1}; sh.step_w > 0.
+__global__ void __launch_bounds__(WG_THREADS, 1)
+    k_wgrad_rows(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmy,
+                 const RowsShape sh, float *__restrict__ partial, int *err) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = tc::smem_u32(smem_raw);
+  const uint32_t x_base = (raw + 1023u) & ~1023u;
+  const uint32_t y_base = x_base + WR_X * WIN_BYTES;
+  const uint32_t ones_base = y_base + WR_Y * WR_Y_BYTES;
+  const uint32_t bar0 = ones_base + WR_Y_BYTES;
+  const uint32_t xfull = bar0, xempty = xfull + 8u * WR_X, yfull = xempty + 8u * WR_X,
+                 yempty = yfull + 8u * WR_Y, done = yempty + 8u * WR_Y, fin = done + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (fin + 8u - raw));
+  volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  {
+    uint32_t *ones = reinterpret_cast<uint32_t *>(smem_raw + (ones_base - raw));
+    for (uint32_t k = threadIdx.x; k < WR_Y_BYTES / 4u; k += blockDim.x) ones[k] = 0x3F803F80u;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < WR_X; ++s) {
+      tc::mbar_init(xfull + 8u * s, 1);
+      tc::mbar_init(xempty + 8u * s, 1);
+    }
+    for (int s = 0; s < WR_Y; ++s) {
+      tc::mbar_init(yfull + 8u * s, 1);
+      tc::mbar_init(yempty + 8u * s, 1);
+    }
+    tc::mbar_init(done, 1);
+    tc::mbar_init(fin, 1);
+    *abort = 0;
+    tc::fence_barrier_init();
+  }
+  if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), 512u);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  int f = (int)((long long)sh.total * blockIdx.x / gridDim.x);
+  const int f1 = (int)((long long)sh.total * (blockIdx.x + 1) / gridDim.x);
+  RowRun run;
+  int wb = 0;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tc::prefetch_map(&tmx);
+      tc::prefetch_map(&tmy);
+      uint32_t nx = 0, ny = 0;  // windows and gradient rows issued
+      bool ok = true;
+      while (ok && bands_next(sh, f, wb, f1, run)) {
+        for (int j = 0; j < run.n + 2; ++j) {
+          const int h = run.h0 + j * sh.sgn * sh.d;
+          const uint32_t xs = nx % WR_X;
+          if (!tc::mbar_wait(xempty + 8u * xs, ((nx / WR_X) & 1u) ^ 1u, abort)) {
+            ok = false;
+            break;
+          }
+          tc::mbar_arrive_expect_tx(xfull + 8u * xs, WIN_BYTES);
+          tc::tma_load_4d(x_base + xs * WIN_BYTES, &tmx, xfull + 8u * xs, 0, run.wb * 128 - WIN_RADIUS,
+                          h - sh.sgn * sh.d, run.b);
+          ++nx;
+          if (j >= run.n) continue;
+          const uint32_t ys = ny % WR_Y;
+          if (!tc::mbar_wait(yempty + 8u * ys, ((ny / WR_Y) & 1u) ^ 1u, abort)) {
+            ok = false;
+            break;
+          }
+          tc::mbar_arrive_expect_tx(yfull + 8u * ys, WR_Y_BYTES);
+          for (int k = 0; k < 2; ++k)
+            tc::tma_load_4d(y_base + ys * WR_Y_BYTES + (uint32_t)k * (WR_Y_BYTES / 2), &tmy, yfull + 8u * ys, 0,
+                            run.wb * 128 + 64 * k, h, run.b);
+          ++ny;
+        }
+      }
+      for (uint32_t k = nx - min(nx, (uint32_t)WR_X); k < nx; ++k)
+        tc::mbar_drain(xfull + 8u * (k % WR_X), (k / WR_X) & 1u);
+      for (uint32_t k = ny - min(ny, (uint32_t)WR_Y); k < ny; ++k)
+        tc::mbar_drain(yfull + 8u * (k % WR_Y), (k / WR_Y) & 1u);
+    }
+  } else if (warp == 1) {
+    // the converged warp runs the loop (descriptors in uniform registers),
+    // lane 0 issues
+    const uint32_t mine = lane == 0 ? 1u : 0u;
+    constexpr uint32_t id64 = tc::idesc_bf16(128, 64, true, true);
+    const uint32_t col = (uint32_t)sh.step_w * 128u;
+    uint32_t nx = 0, q0 = 0;
+    bool ok = true, first = true;
+    while (ok && bands_next(sh, f, wb, f1, run)) {
+      const int n = run.n;
+      for (int j = 0; j < n + 2; ++j, ++nx) {
+        const uint32_t xs = nx % WR_X, qj = q0 + (uint32_t)j;
+        if (!tc::mbar_wait(xfull + 8u * xs, (nx / WR_X) & 1u, abort) ||
+            (j < n && !tc::mbar_wait(yfull + 8u * (qj % WR_Y), (qj / WR_Y) & 1u, abort))) {
+          ok = false;
+          break;
+        }
+        tc::fence_after_sync();
+        const int lo = max(0, j - 2);
+        const uint32_t cnt = (uint32_t)(min(n - 1, j) - lo + 1);
+        const uint32_t ys = (q0 + (uint32_t)lo) % WR_Y;
+        // gradient rows lo .. lo + cnt - 1 = tap rows j - lo, ...; those
+        // beyond the ring's end take a second instruction
+        const uint32_t n1 = min(cnt, (uint32_t)WR_Y - ys), n2 = cnt - n1;
+        const uint32_t d0 = tmem + 64u * (uint32_t)(2 - (j - lo));
+        const uint32_t a0 = x_base + xs * WIN_BYTES + WIN_RADIUS * 128u - col;
+        const uint64_t ad0 = tc::sdesc(a0, col, 1024u);
+        const uint64_t ad1 = tc::sdesc(a0 + 2u * col, ones_base - (a0 + 2u * col), 1024u);
+        const uint64_t bd1 = tc::sdesc(y_base + ys * WR_Y_BYTES, WR_Y_BYTES, 1024u);
+        const uint64_t bd2 = tc::sdesc(y_base, WR_Y_BYTES, 1024u);
+        const uint32_t id1 = id64 + ((n1 - 1u) << 20), id2 = id64 + ((n2 - 1u) << 20);
+        if (first && j <= 2) {
+          // row lo = 0 meets tap row j for the first time: its first
+          // instruction starts the accumulator
+          for (uint32_t p = 0; p < 2; ++p) {
+            const uint64_t ad = p ? ad1 : ad0;
+            const uint32_t d = d0 + 192u * p;
+            for (uint32_t k = 0; k < 8; ++k)
+              for (uint32_t g = 0; g < cnt; ++g) {
+                const uint64_t bd = g < n1 ? bd1 + g * (WR_Y_BYTES / 16u) : bd2 + (g - n1) * (WR_Y_BYTES / 16u);
+                tc::mma_bf16_warp(mine, d + 64u * g, ad + 128u * k, bd + 128u * k, id64,
+                                  (g == 0 && k == 0) ? 0u : 1u);
+              }
+          }
+        } else if (n2 == 0u) {
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) {
+            tc::mma_bf16_warp(mine, d0, ad0 + 128u * k, bd1 + 128u * k, id1, 1u);
+            tc::mma_bf16_warp(mine, d0 + 192u, ad1 + 128u * k, bd1 + 128u * k, id1, 1u);
+          }
+        } else {
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) {
+            tc::mma_bf16_warp(mine, d0, ad0 + 128u * k, bd1 + 128u * k, id1, 1u);
+            tc::mma_bf16_warp(mine, d0 + 64u * n1, ad0 + 128u * k, bd2 + 128u * k, id2, 1u);
+            tc::mma_bf16_warp(mine, d0 + 192u, ad1 + 128u * k, bd1 + 128u * k, id1, 1u);
+            tc::mma_bf16_warp(mine, d0 + 192u + 64u * n1, ad1 + 128u * k, bd2 + 128u * k, id2, 1u);
+          }
+        }
+        tc::mma_commit_warp(mine, xempty + 8u * xs);
+        if (j >= 2) tc::mma_commit_warp(mine, yempty + 8u * ((qj - 2u) % WR_Y));
+      }
+      q0 += (uint32_t)n;
+      first = false;
+    }
+    if (ok) tc::mma_commit_warp(mine, done);
+    tc::mma_commit_warp(mine, fin);
+    tc::mbar_drain(fin, 0);
+  } else {
+    const int row = (warp & 3) * 32 + lane;
+    if (tc::mbar_wait(done, 0, abort)) {
+      tc::fence_after_sync();
+      for (int p = 0; p < 2; ++p) {
+        const int c = 2 * p + (row >> 6);  // tap column; 3: the all-ones block
+        for (int r = 0; r < 3; ++r) {
+          const int atom = c < 3 ? 3 * r + c : 9;
+          float *dst = partial + ((size_t)blockIdx.x * WR_ATOMS + atom) * 4096u + (row & 63);
+          const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 192u * (uint32_t)p + 64u * (uint32_t)(2 - r);
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            float v[16];
+            tc::tmem_ld16(taddr + (uint32_t)c0, v);
+            if (c < 3 || r == 1) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) dst[(size_t)(c0 + i) * 64] = v[i];
+            }
+          }
+        }
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 512u);
   }
   if (threadIdx.x == 0 && *abort) atomicOr(err, 2);
 }
