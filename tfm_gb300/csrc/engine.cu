@@ -709,18 +709,37 @@ struct Engine {
   }
 
   // -------------------------------------------------------------- launches
+  // Kernels of a captured chain of steps are programmatic dependents of the
+  // one before (pdl_wait): the next kernel is launched while the last CTAs of
+  // this one run. The first kernel of a chain, and every kernel outside one,
+  // waits as a stream orders it.
+  bool chained = false;
+  template <typename... P, typename... A>
+  void launch(void (*kernel)(P...), unsigned grid, unsigned block, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    CK(cudaLaunchKernelEx(&c, kernel, P(args)...));
+    if (chain_open) chained = true;
+    kcount += 1;
+  }
+  bool chain_open = false;  // capturing a chain
+
   void launch_scan(bool bump) {
-    k_scan_reduce<<<nblk, SCAN_THREADS, 0, stream>>>(counts.p, bsum.p);
-    k_scan_top<<<1, SCAN_TOP_THREADS, 0, stream>>>(bsum.p, nblk, d_step.p, bump ? 1 : 0);
-    k_scan_apply<<<nblk, SCAN_THREADS, 0, stream>>>(counts.p, bsum.p, start.p, nc, nblk);
-    kcount += 3;
+    launch(k_scan_reduce, nblk, SCAN_THREADS, counts.p, bsum.p);
+    launch(k_scan_top, 1, SCAN_TOP_THREADS, bsum.p, nblk, d_step.p, bump ? 1 : 0);
+    launch(k_scan_apply, nblk, SCAN_THREADS, counts.p, bsum.p, start.p, nc, nblk);
   }
 
   void launch_scatter(const float4 *src) {
-    k_scatter<<<(unsigned)htiles.size(), tile, 0, stream>>>(
-        d_tiles.p, d_sys.p, src, rank.p, start.p, sorted.p,
-        par.pair_kernel >= 2 ? fs.p : nullptr, counts.p, d_err.p);
-    kcount += 1;
+    launch(k_scatter, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, src, rank.p, start.p,
+           sorted.p, par.pair_kernel >= 2 ? fs.p : nullptr, counts.p, d_err.p);
   }
 
   // Typed layout (pair_kernel 4): A beads and the others sorted into separate
@@ -777,17 +796,17 @@ struct Engine {
   void launch_typed(unsigned nt) {
     const int L = (tile * pair_lanes() <= 512) ? pair_lanes() : 1;
     if (L == 8)
-      k_pair_typed_lanes<MODE, RHH, RX, 8><<<nt, (unsigned)(tile * 8), 0, stream>>>(
-          d_tiles.p, d_sys.p, ff, sorted.p, start.p, fs.p);
+      launch(k_pair_typed_lanes<MODE, RHH, RX, 8>, nt, (unsigned)(tile * 8), d_tiles.p, d_sys.p, ff,
+             sorted.p, start.p, fs.p);
     else if (L == 4)
-      k_pair_typed_lanes<MODE, RHH, RX, 4><<<nt, (unsigned)(tile * 4), 0, stream>>>(
-          d_tiles.p, d_sys.p, ff, sorted.p, start.p, fs.p);
+      launch(k_pair_typed_lanes<MODE, RHH, RX, 4>, nt, (unsigned)(tile * 4), d_tiles.p, d_sys.p, ff,
+             sorted.p, start.p, fs.p);
     else if (L == 2)
-      k_pair_typed_lanes<MODE, RHH, RX, 2><<<nt, (unsigned)(tile * 2), 0, stream>>>(
-          d_tiles.p, d_sys.p, ff, sorted.p, start.p, fs.p);
+      launch(k_pair_typed_lanes<MODE, RHH, RX, 2>, nt, (unsigned)(tile * 2), d_tiles.p, d_sys.p, ff,
+             sorted.p, start.p, fs.p);
     else
-      k_pair_typed<MODE, RHH, RX><<<nt, tile, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                           start.p, fs.p);
+      launch(k_pair_typed<MODE, RHH, RX>, nt, tile, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+             fs.p);
   }
 
   template <int MODE>
@@ -805,61 +824,59 @@ struct Engine {
           launch_typed<MODE, 2, 2>(nt);
           break;
         default:  // systems gridded differently: each system's own reaches
-          k_pair_typed<MODE, 0, 0><<<nt, tile, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+          launch(k_pair_typed<MODE, 0, 0>, nt, tile, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+                 fs.p);
       }
     } else if (par.pair_kernel == 0)
-      k_pair<MODE><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                                  start.p, fs.p);
+      launch(k_pair<MODE>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+             fs.p);
     else if (par.pair_kernel == 3 && par.reach == 2)
-      k_pair_flat<MODE, 2><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff,
-                                                                          sorted.p, start.p, fs.p);
+      launch(k_pair_flat<MODE, 2>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p,
+             start.p, fs.p);
     else if (par.pair_kernel == 3)
-      k_pair_flat<MODE><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff,
-                                                                       sorted.p, start.p, fs.p);
+      launch(k_pair_flat<MODE>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p,
+             start.p, fs.p);
     else if (par.pair_kernel == 2 && pair_lanes() > 1 && uniform_reach() > 0 &&
              tile * pair_lanes() <= 512) {
       const unsigned bs = (unsigned)(tile * pair_lanes());
       const int r = uniform_reach();
       if (pair_lanes() == 2 && r == 2)
-        k_pair_half_lanes<MODE, 2, 2><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 2, 2>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
       else if (pair_lanes() == 2)
-        k_pair_half_lanes<MODE, 1, 2><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 1, 2>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
       else if (pair_lanes() == 8 && r == 2)
-        k_pair_half_lanes<MODE, 2, 8><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 2, 8>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
       else if (pair_lanes() == 8)
-        k_pair_half_lanes<MODE, 1, 8><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 1, 8>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
       else if (r == 2)
-        k_pair_half_lanes<MODE, 2, 4><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 2, 4>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
       else
-        k_pair_half_lanes<MODE, 1, 4><<<nt, bs, 0, stream>>>(d_tiles.p, d_sys.p, ff, sorted.p,
-                                                             start.p, fs.p);
+        launch(k_pair_half_lanes<MODE, 1, 4>, nt, bs, d_tiles.p, d_sys.p, ff, sorted.p, start.p,
+               fs.p);
     } else if (par.pair_kernel == 2 && uniform_reach() == 2)
-      k_pair_half<MODE, 2><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff,
-                                                                          sorted.p, start.p, fs.p);
+      launch(k_pair_half<MODE, 2>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p,
+             start.p, fs.p);
     else if (par.pair_kernel == 2 && uniform_reach() == 1)
-      k_pair_half<MODE, 1><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff,
-                                                                          sorted.p, start.p, fs.p);
+      launch(k_pair_half<MODE, 1>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p,
+             start.p, fs.p);
     else if (par.pair_kernel == 2)  // mixed: each system's own stencil reach
-      k_pair_half<MODE, 0><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, ff,
-                                                                          sorted.p, start.p, fs.p);
+      launch(k_pair_half<MODE, 0>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, sorted.p,
+             start.p, fs.p);
     else
-      k_pair_cells<MODE><<<(unsigned)hctiles.size(), PAIR_WARPS * 32, 0, stream>>>(
-          d_ctiles.p, d_sys.p, ff, sorted.p, start.p, fs.p);
-    kcount += 1;
+      launch(k_pair_cells<MODE>, (unsigned)hctiles.size(), PAIR_WARPS * 32, d_ctiles.p, d_sys.p, ff,
+             sorted.p, start.p, fs.p);
   }
 
   template <int STAGE, int MODE>
   void launch_update() {
-    k_update<STAGE, MODE><<<(unsigned)htiles.size(), tile, 0, stream>>>(
-        d_tiles.p, d_sys.p, ff, pos.p, er.p, fbuf.p, rnb.p, fs.p, rank.p, counts.p, lbs_sorted.p,
-        lbs_start.p, d_step.p, d_err.p);
-    kcount += 1;
+    launch(k_update<STAGE, MODE>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, pos.p,
+           er.p, fbuf.p, rnb.p, fs.p, rank.p, counts.p, lbs_sorted.p, lbs_start.p, d_step.p,
+           d_err.p);
   }
 
   ContactArgs contact_args(bool do_map, bool do_ps, bool do_ovl) {
@@ -891,23 +908,21 @@ struct Engine {
   void launch_contacts_args(const ContactArgs &a) {
     const int r = uniform_reach();
     if (r == 1)
-      k_contacts_half<1><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, sorted.p,
-                                                                    start.p, a);
+      launch(k_contacts_half<1>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
     else if (r == 2)
-      k_contacts_half<2><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, sorted.p,
-                                                                    start.p, a);
+      launch(k_contacts_half<2>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
     else
-      k_contacts_half<0><<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, sorted.p,
-                                                                    start.p, a);
-    kcount += 1;
+      launch(k_contacts_half<0>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
   }
 
   void launch_contacts() { launch_contacts_args(contact_args(true, true, false)); }
 
   void launch_observe() {
-    k_observe<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p,
-                                                             CCP_RCO / 2.0f, obs.p);
-    kcount += 1;
+    launch(k_observe, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, pos.p, CCP_RCO / 2.0f,
+           obs.p);
   }
 
   void launch_observe_sorted(bool with_sdist) {
@@ -970,6 +985,12 @@ struct Engine {
     cudaGraph_t g;
     uint64_t k0 = kcount;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    struct Chain {  // the launches below are programmatic dependents
+      Engine *e;
+      explicit Chain(Engine *e_) : e(e_) { e->chain_open = true; }
+      ~Chain() { e->chain_open = e->chained = false; }
+    };
+    auto chain = std::make_unique<Chain>(this);
     if (mode >= FUSED_KIND) launch_fused_steps(mode - FUSED_KIND, n, obs);
     for (int k = 0; k < n && mode < FUSED_KIND; ++k) {
       if (mode == MODE_DST)
@@ -977,6 +998,7 @@ struct Engine {
       else
         launch_step<MODE_ICG>(false);
     }
+    chain.reset();
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     graph_kernels[key] = kcount - k0;  // captured, not executed: counted per replay
     kcount = k0;

@@ -67,14 +67,6 @@ struct FusedArgs {
   int n_cells;
 };
 
-// Programmatic dependent launch: the next kernel's CTAs may start (and read
-// their constant tables) while this one runs; they wait here until every
-// write of the kernel before is visible.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 __device__ __forceinline__ int fused_cell(float4 p, const FusedGrid &g, bool &esc) {
   const int n = g.cps - 2;
   const int x = cell_coord(p.x, g.inv_csl, n, esc), y = cell_coord(p.y, g.inv_csl, n, esc),

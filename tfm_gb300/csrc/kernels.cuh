@@ -45,6 +45,14 @@ struct Tile {
 
 // ------------------------------------------------------------------ helpers
 
+// Programmatic dependent launch: the next kernel's CTAs may start (and read
+// their constant tables) while this one runs; they wait here until every
+// write of the kernel before is visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t wbits(float4 p) { return __float_as_uint(p.w); }
 
 // Integer cell coordinate along one axis of a grid centred at the origin with
@@ -330,6 +338,8 @@ __device__ __forceinline__ uint32_t cell_add(uint32_t *counts, int c, int *err) 
 __global__ void k_count(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
                         const float4 *__restrict__ pos, uint32_t *__restrict__ counts,
                         uint32_t *__restrict__ rank, int *__restrict__ err) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int i = t.begin + threadIdx.x;
@@ -379,6 +389,8 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *total)
 // SCAN_CHUNK cells (zeros beyond n_cells).
 __global__ void __launch_bounds__(SCAN_THREADS)
     k_scan_reduce(const uint32_t *__restrict__ counts, uint32_t *__restrict__ block_sums) {
+  pdl_wait();
+  pdl_trigger();
   static_assert(SCAN_ITEMS == 16, "one uint4 of byte counts per thread");
   const uint4 q = reinterpret_cast<const uint4 *>(counts)[(size_t)blockIdx.x * SCAN_THREADS +
                                                          threadIdx.x];
@@ -400,6 +412,8 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 // scan opens a new Heun step (bump != 0).
 __global__ void __launch_bounds__(SCAN_TOP_THREADS)
     k_scan_top(uint32_t *__restrict__ block_sums, int nb, unsigned long long *step, int bump) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ uint32_t tot;
   uint32_t carry = 0;
   for (int b0 = 0; b0 < nb; b0 += SCAN_TOP_THREADS) {
@@ -422,6 +436,8 @@ __global__ void __launch_bounds__(SCAN_TOP_THREADS)
 __global__ void __launch_bounds__(SCAN_THREADS)
     k_scan_apply(const uint32_t *__restrict__ counts, const uint32_t *__restrict__ block_sums,
                  uint32_t *__restrict__ start, int n_cells, int nb) {
+  pdl_wait();
+  pdl_trigger();
   const uint4 q = reinterpret_cast<const uint4 *>(counts)[(size_t)blockIdx.x * SCAN_THREADS +
                                                          threadIdx.x];
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -454,6 +470,8 @@ __global__ void k_scatter(const Tile *__restrict__ tiles, const SysDesc *__restr
                           const uint32_t *__restrict__ start, float4 *__restrict__ sorted,
                           float4 *__restrict__ fs_clear, uint32_t *__restrict__ counts,
                           int *__restrict__ err) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int i = t.begin + threadIdx.x;
@@ -521,6 +539,8 @@ __global__ void __launch_bounds__(256)
     k_pair(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys, ForceField ff,
            const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
            float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int slot = t.begin + threadIdx.x;
@@ -633,6 +653,8 @@ __global__ void __launch_bounds__(256, 8)
     k_pair_half(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys, ForceField ff,
                 const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                 float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int slot = t.begin + threadIdx.x;
@@ -756,6 +778,8 @@ __global__ void __launch_bounds__(256, 8)
     k_pair_typed(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys, ForceField ff,
                  const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                  float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int slot = t.begin + threadIdx.x;
@@ -798,6 +822,8 @@ __global__ void __launch_bounds__(512)
     k_pair_half_lanes(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
                       ForceField ff, const float4 *__restrict__ sorted,
                       const uint32_t *__restrict__ start, float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   const int sub = threadIdx.x % L;
@@ -871,6 +897,8 @@ __global__ void __launch_bounds__(512)
     k_pair_typed_lanes(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
                        ForceField ff, const float4 *__restrict__ sorted,
                        const uint32_t *__restrict__ start, float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   const int sub = threadIdx.x % L;
@@ -961,6 +989,8 @@ __global__ void __launch_bounds__(256)
     k_pair_flat(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys, ForceField ff,
                 const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                 float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int slot = t.begin + threadIdx.x;
@@ -1008,6 +1038,8 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, 4)
     k_pair_cells(const Tile *__restrict__ ctiles, const SysDesc *__restrict__ sys, ForceField ff,
                  const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                  float4 *__restrict__ fs) {
+  pdl_wait();
+  pdl_trigger();
   // cell starts of the 9 neighbour rows over x in [xb - 1, xb + PAIR_WARPS + 1],
   // staged once for the CTA (all warps reach the barrier before any returns)
   __shared__ uint32_t s_start[9][PAIR_WARPS + 4];
@@ -1211,6 +1243,8 @@ __global__ void __launch_bounds__(256, 7)
              uint32_t *__restrict__ counts,
              const float4 *__restrict__ lbs, const uint32_t *__restrict__ lbs_start,
              const unsigned long long *__restrict__ step, int *__restrict__ err) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int i = t.begin + threadIdx.x;
@@ -1450,6 +1484,8 @@ __global__ void __launch_bounds__(256)
     k_contacts_half(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
                     const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                     ContactArgs a) {
+  pdl_wait();
+  pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
   int slot = t.begin + threadIdx.x;
@@ -1501,6 +1537,8 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 __global__ void __launch_bounds__(OBS_WARPS * 32)
     k_observe(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
               const float4 *__restrict__ pos, float bead_r, double *__restrict__ acc) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float hist[OBS_WARPS][3 * N_SHELLS];
   __shared__ double sums[4];
   __shared__ float rb[N_SHELLS];
