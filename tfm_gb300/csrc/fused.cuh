@@ -147,9 +147,10 @@ __device__ __forceinline__ float3 fused_lbs(float4 x, const SysDesc &s, const Fo
                                             const uint32_t *__restrict__ lbs_start, int first,
                                             int stride) {
   float3 f = make_float3(0.0f, 0.0f, 0.0f);
-  float d = sqrtf(x.x * x.x + x.y * x.y + x.z * x.z);
+  float d2 = x.x * x.x + x.y * x.y + x.z * x.z;
   float m = ff.lco * 1.001f + 1e-4f;
-  if (d < s.lbs_rmin - m || d > s.lbs_rmax + m) return f;  // no site within reach
+  float lo = fmaxf(s.lbs_rmin - m, 0.0f), hi = s.lbs_rmax + m;
+  if (d2 < lo * lo || d2 > hi * hi) return f;  // no site within reach
   bool esc = false;
   int xl = cell_coord(x.x - m, s.inv_csl, s.cps, esc), xh = cell_coord(x.x + m, s.inv_csl, s.cps, esc);
   int yl = cell_coord(x.y - m, s.inv_csl, s.cps, esc), yh = cell_coord(x.y + m, s.inv_csl, s.cps, esc);
@@ -324,14 +325,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
     }
     F = bonded_force_at([&](int j) { return j < io ? nb[j - io + 2] : nb[j - io + 1]; }, io, xi, end,
                         ff);
-    float3 vw;
-    float gh, gl;
-    if (wall_vector<MODE_DST>(make_float3(xi.x, xi.y, xi.z), s, vw, gh, gl)) {
-      const float cw = wall_coef<MODE_DST>(gh, gl, ff);
-      F.x += cw * vw.x;
-      F.y += cw * vw.y;
-      F.z += cw * vw.z;
-    }
+    add_wall<MODE_DST>(xi, s, ff, F);
   }
   __syncthreads();
   if (!mine) return;

@@ -139,20 +139,25 @@ constexpr float LJ_Z2_HI = 1.259921074e+00f;
 constexpr float LJ_Z2_LO = -2.401870169e-08f;
 constexpr float LJ_Z2_SQ = 1.587401032e+00f;
 
-// d^2 - 2^(1/3) for the pair vector (dx, dy, dz), |components| < 2, without
-// cancellation: each component is split as x = xh + xl with xh on a 2^-10
-// grid (rounded by adding and subtracting 1.5 * 2^13), so xh^2 and the sum of
-// the three are exact in FP32 and the sum minus 2^(1/3) is exact (Sterbenz)
-// for d^2 within a factor 2 of it; x^2 - xh^2 = xl (xh + x) is small.
-__device__ __forceinline__ float lj_zero_gap(float dx, float dy, float dz) {
+// d^2 - (kh + kl) for the vector (dx, dy, dz) without cancellation where d^2 is
+// within a factor 2 of kh < 8: each component is split as x = xh + xl with xh on
+// a 2^-10 grid (rounded by adding and subtracting 1.5 * 2^13), so xh^2 and the
+// sum of the three are exact in FP32 and the sum minus kh is exact (Sterbenz);
+// x^2 - xh^2 = xl (xh + x) is small. Elsewhere nothing cancels.
+__device__ __forceinline__ float sq3_gap(float dx, float dy, float dz, float kh, float kl) {
   const float M = 12288.0f;
   float xh = __fsub_rn(__fadd_rn(dx, M), M), yh = __fsub_rn(__fadd_rn(dy, M), M),
         zh = __fsub_rn(__fadd_rn(dz, M), M);
   float sh = __fmaf_rn(zh, zh, __fmaf_rn(yh, yh, __fmul_rn(xh, xh)));
   float lo = __fmaf_rn(__fsub_rn(dx, xh), __fadd_rn(xh, dx),
                        __fmaf_rn(__fsub_rn(dy, yh), __fadd_rn(yh, dy),
-                                 __fmaf_rn(__fsub_rn(dz, zh), __fadd_rn(zh, dz), -LJ_Z2_LO)));
-  return __fadd_rn(__fsub_rn(sh, LJ_Z2_HI), lo);
+                                 __fmaf_rn(__fsub_rn(dz, zh), __fadd_rn(zh, dz), -kl)));
+  return __fadd_rn(__fsub_rn(sh, kh), lo);
+}
+
+// d^2 - 2^(1/3), the gap to the Lennard-Jones force's zero.
+__device__ __forceinline__ float lj_zero_gap(float dx, float dy, float dz) {
+  return sq3_gap(dx, dy, dz, LJ_Z2_HI, LJ_Z2_LO);
 }
 
 // Lennard-Jones coefficient 24 e (2 / d^14 - 1 / d^8) = 24 e d^-8 (2 d^-6 - 1)
@@ -296,6 +301,26 @@ __device__ __forceinline__ float wall_coef(float gh, float gl, const ForceField 
   float m = __fsub_rn(__fsub_rn(2.0f, p2), lo6);
   float i6 = i4 * i2;
   return 24.0f * e * m * (i6 * i6 * i2);  // 1 / g^14
+}
+
+// Wall force of a bead, added to F. Inside a bare sphere the beads further from
+// the wall than its cutoff, most of them, are told by their squared distance
+// (with a margin for its rounding): gap and coefficient take some 200
+// instructions of the update pass's 800 to 1050, and a warp skips them when all
+// its beads are inside.
+template <int MODE>
+__device__ __forceinline__ void add_wall(float4 x, const SysDesc &s, const ForceField &ff, float3 &F) {
+  if (MODE == MODE_ICG || s.R_o == 0.0f) {
+    const float in = s.R_n * (1.0f - 1e-5f) - (MODE == MODE_ICG ? ICG_WALL_RC : ff.rc_w) - 1e-3f;
+    if (in > 0.0f && x.x * x.x + x.y * x.y + x.z * x.z < in * in) return;
+  }
+  float3 v;
+  float gh, gl;
+  if (!wall_vector<MODE>(make_float3(x.x, x.y, x.z), s, v, gh, gl)) return;
+  const float c = wall_coef<MODE>(gh, gl, ff);
+  F.x += c * v.x;
+  F.y += c * v.y;
+  F.z += c * v.z;
 }
 
 // Truncated standard normals for one bead and step: three Box-Muller normals
@@ -1110,9 +1135,10 @@ __device__ __forceinline__ float3 lbs_force(float4 x, const SysDesc &s, const Fo
                                             const float4 *__restrict__ lbs,
                                             const uint32_t *__restrict__ lbs_start) {
   float3 f = make_float3(0.0f, 0.0f, 0.0f);
-  float d = sqrtf(x.x * x.x + x.y * x.y + x.z * x.z);
+  float d2 = x.x * x.x + x.y * x.y + x.z * x.z;
   float m = ff.lco * 1.001f + 1e-4f;
-  if (d < s.lbs_rmin - m || d > s.lbs_rmax + m) return f;  // no site within reach
+  float lo = fmaxf(s.lbs_rmin - m, 0.0f), hi = s.lbs_rmax + m;
+  if (d2 < lo * lo || d2 > hi * hi) return f;  // no site within reach
   bool esc = false;
   int xl = cell_coord(x.x - m, s.inv_csl, s.cps, esc), xh = cell_coord(x.x + m, s.inv_csl, s.cps, esc);
   int yl = cell_coord(x.y - m, s.inv_csl, s.cps, esc), yh = cell_coord(x.y + m, s.inv_csl, s.cps, esc);
@@ -1180,14 +1206,14 @@ __device__ __forceinline__ float3 bonded_force_at(Load X, int i, float4 xi, int 
   if (e1) {
     float cx = v1.x * two_sum_err(xi.x, -xm1.x, v1.x) + v1.y * two_sum_err(xi.y, -xm1.y, v1.y) +
                v1.z * two_sum_err(xi.z, -xm1.z, v1.z);
-    float s1 = __fadd_rn(sq3_minus(v1.x, v1.y, v1.z, lh, ll), 2.0f * cx);
+    float s1 = __fadd_rn(sq3_gap(v1.x, v1.y, v1.z, lh, ll), 2.0f * cx);
     float d1 = sqrtf(v1.x * v1.x + v1.y * v1.y + v1.z * v1.z);
     ke1 = ff.k_e * (s1 / (d1 + ff.l_0)) * il1;
   }
   if (e2) {
     float cx = v2.x * two_sum_err(xp1.x, -xi.x, v2.x) + v2.y * two_sum_err(xp1.y, -xi.y, v2.y) +
                v2.z * two_sum_err(xp1.z, -xi.z, v2.z);
-    float s2 = __fadd_rn(sq3_minus(v2.x, v2.y, v2.z, lh, ll), 2.0f * cx);
+    float s2 = __fadd_rn(sq3_gap(v2.x, v2.y, v2.z, lh, ll), 2.0f * cx);
     float d2 = sqrtf(v2.x * v2.x + v2.y * v2.y + v2.z * v2.z);
     ke2 = ff.k_e * (s2 / (d2 + ff.l_0)) * il2;
   }
@@ -1269,14 +1295,7 @@ __global__ void __launch_bounds__(256, 7)
   F.y += fb.y;
   F.z += fb.z;
 
-  float3 vw;
-  float gh, gl;
-  if (wall_vector<MODE>(make_float3(xi.x, xi.y, xi.z), s, vw, gh, gl)) {
-    float cw = wall_coef<MODE>(gh, gl, ff);
-    F.x += cw * vw.x;
-    F.y += cw * vw.y;
-    F.z += cw * vw.z;
-  }
+  add_wall<MODE>(xi, s, ff, F);
   if (MODE == MODE_DST && (fl & BF_LAD) && s.n_lbs > 0) {
     float3 fl3 = lbs_force(xi, s, ff, lbs, lbs_start);
     F.x += fl3.x;
@@ -1343,14 +1362,7 @@ __global__ void k_total_force(const Tile *__restrict__ tiles, const SysDesc *__r
   F.x += fb.x;
   F.y += fb.y;
   F.z += fb.z;
-  float3 vw;
-  float gh, gl;
-  if (wall_vector<MODE>(make_float3(xi.x, xi.y, xi.z), s, vw, gh, gl)) {
-    float cw = wall_coef<MODE>(gh, gl, ff);
-    F.x += cw * vw.x;
-    F.y += cw * vw.y;
-    F.z += cw * vw.z;
-  }
+  add_wall<MODE>(xi, s, ff, F);
   if (MODE == MODE_DST && (wbits(xi) & BF_LAD) && s.n_lbs > 0) {
     float3 fl3 = lbs_force(xi, s, ff, lbs, lbs_start);
     F.x += fl3.x;
