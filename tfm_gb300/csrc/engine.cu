@@ -291,10 +291,16 @@ struct Engine {
     }
     need_cut = std::max({ff.rc_att, ff.rc_rep, ff.rc_icg, p.contact_cutoff, ff.mis});
     for (auto &d : hsys) d.reach = (d.csl >= need_cut) ? 1 : 2;
-    // batches too small to fill the GPU: tiles of 64 beads, eight lanes per
-    // bead in the pair pass (pair_lanes); measured on single ccp systems of
-    // 1024-8192 beads 8-12 % faster per Heun step than tiles of 128 with four
-    tile = (nb < SMALL_BATCH) ? 64 : TILE;
+    // Tiles of 64 beads: batches too small to fill the GPU (with eight lanes
+    // per bead in the pair pass, pair_lanes: single ccp systems of 1024-8192
+    // beads 8-12 % faster per Heun step than tiles of 128 with four), and
+    // batches of a few waves of CTAs, whose end is ragged with larger ones. us
+    // per step with tiles of 128 / 64, baseline: 60000 beads 62.4 / 58.1, 50 x
+    // 1024 68.4 / 64.1, 64 x 2000 104.8 / 99.0, 30 x 7000 132.6 / 128.6, but
+    // 131072 in one system 84.0 / 89.3 (its A beads come first and fill the
+    // ragged end's place), 512 replicas 898 / 915; ccp 40 x 4000 85.5 / 83.0,
+    // 128 x 1024 77.6 / 78.4.
+    tile = (nb < SMALL_BATCH || (nb < 262144 && (ns > 1 || nb < 100000))) ? 64 : TILE;
     build_tiles();
     nblk = (nc + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK;
 
