@@ -152,6 +152,8 @@ struct Engine {
   DevBuf<int32_t> d_chain_of, d_chain_first, d_chain_len, d_chain_ps_off, d_chain_smax;
   DevBuf<int32_t> map, ps;
   DevBuf<double> obs, ds;
+  std::vector<long long> sdist_off;  // first CTA of every chain in k_sdist, and the total
+  DevBuf<long long> d_sdist_off;
   // ccp-analyze's outputs (analysis.h): per-frame sums of the observables and
   // the nematic order / nucleus fraction sums of the frame being analysed
   Analysis ana;
@@ -911,17 +913,33 @@ struct Engine {
     return r;
   }
 
+  template <int REACH>
+  void launch_contacts_reach(const ContactArgs &a) {
+    // as many lanes a bead as the pair pass takes by default
+    const int by_size = nb < SMALL_BATCH ? 8 : (nb < 65536 ? 4 : (nb < 262144 ? 2 : 1));
+    const unsigned nt = (unsigned)htiles.size();
+    if (by_size == 8 && tile * 8 <= 512)
+      launch(k_contacts_half<REACH, 8>, nt, (unsigned)(tile * 8), d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
+    else if (by_size >= 4 && tile * 4 <= 512)
+      launch(k_contacts_half<REACH, 4>, nt, (unsigned)(tile * 4), d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
+    else if (by_size >= 2)
+      launch(k_contacts_half<REACH, 2>, nt, (unsigned)(tile * 2), d_tiles.p, d_sys.p, sorted.p,
+             start.p, a);
+    else
+      launch(k_contacts_half<REACH, 1>, nt, (unsigned)tile, d_tiles.p, d_sys.p, sorted.p, start.p,
+             a);
+  }
+
   void launch_contacts_args(const ContactArgs &a) {
     const int r = uniform_reach();
     if (r == 1)
-      launch(k_contacts_half<1>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
-             start.p, a);
+      launch_contacts_reach<1>(a);
     else if (r == 2)
-      launch(k_contacts_half<2>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
-             start.p, a);
+      launch_contacts_reach<2>(a);
     else
-      launch(k_contacts_half<0>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, sorted.p,
-             start.p, a);
+      launch_contacts_reach<0>(a);
   }
 
   void launch_contacts() { launch_contacts_args(contact_args(true, true, false)); }
@@ -935,20 +953,18 @@ struct Engine {
     launch_contacts();
     launch_observe();
     if (with_sdist) {
-      int smax = 0, lmax = 0;
-      for (int c = 0; c < nch; ++c) {
-        smax = std::max(smax, chain_smax[c]);
-        lmax = std::max(lmax, chain_len[c]);
+      if (!d_sdist_off.p) {
+        sdist_off.assign(1, 0);
+        for (int c = 0; c < nch; ++c)
+          sdist_off.push_back(sdist_off.back() + sdist_tiles(chain_len[c], chain_smax[c]));
+        d_sdist_off.alloc(sdist_off.size());
+        CK(cudaMemcpyAsync(d_sdist_off.p, sdist_off.data(), sizeof(long long) * sdist_off.size(),
+                           cudaMemcpyHostToDevice, stream));
       }
-      if (smax > 0) {
-        for (int c = 0; c < nch; ++c) {
-          dim3 grid((chain_smax[c] + 127) / 128, (chain_len[c] + SDIST_PCHUNK - 1) / SDIST_PCHUNK);
-          if (chain_smax[c] == 0) continue;
-          k_sdist<<<grid, 128, 0, stream>>>(pos.p, d_chain_first.p, d_chain_len.p,
-                                            d_chain_ps_off.p, d_chain_smax.p, c, ds.p);
-          kcount += 1;
-        }
-      }
+      const long long total = sdist_off.back(), most = 1ll << 30;  // CTAs of a launch
+      for (long long t = 0; t < total; t += most)
+        launch(k_sdist, (unsigned)std::min(most, total - t), SDIST_SEPS, pos.p, d_chain_first.p,
+               d_chain_len.p, d_chain_ps_off.p, d_chain_smax.p, d_sdist_off.p, nch, t, ds.p);
     }
   }
 

@@ -1440,45 +1440,31 @@ __device__ __forceinline__ void contact_pair(float4 p, const ContactBead &bi, fl
   }
 }
 
-// Forward half of the (2R+1)^3 stencil in the grid starting at cell g0 (the
-// own cell after `slot` and the +x cells, the +y rows, the +z layers), or
-// the full stencil (FULL) of that grid.
-template <bool FULL>
-__device__ __forceinline__ void contact_rows(float4 p, const ContactBead &bi, int slot, CellXYZ c,
-                                             int g0, int R, const SysDesc &s,
+// Rows sub, sub + L, ... of the forward half of the (2R+1)^3 stencil in the grid
+// starting at cell g0 (row 0: the own cell after `slot` and the +x cells, then
+// the +y rows, the +z layers), or of the full stencil (FULL) of that grid.
+template <bool FULL, int L>
+__device__ __forceinline__ void contact_rows(float4 p, const ContactBead &bi, int slot, int sub,
+                                             CellXYZ c, int g0, int R, const SysDesc &s,
                                              const float4 *__restrict__ sorted,
                                              const uint32_t *__restrict__ start,
                                              const ContactArgs &a, unsigned long long &novl) {
-  const int cps = s.cps;
+  const int cps = s.cps, W = 2 * R + 1;
   const int x0 = max(c.x - R, 0), x1 = min(c.x + R, cps - 1);
-  if (FULL) {
-    for (int z = max(c.z - R, 0); z <= min(c.z + R, cps - 1); ++z)
-      for (int y = max(c.y - R, 0); y <= min(c.y + R, cps - 1); ++y) {
-        int row = g0 + (z * cps + y) * cps;
-        for (uint32_t k = __ldg(&start[row + x0]), e = __ldg(&start[row + x1 + 1]); k < e; ++k)
-          contact_pair(p, bi, __ldg(&sorted[k]), s, a, novl);
-      }
-    return;
-  }
-  {
-    int row = g0 + (c.z * cps + c.y) * cps;
-    for (uint32_t k = slot + 1, e = __ldg(&start[row + x1 + 1]); k < e; ++k)
-      contact_pair(p, bi, __ldg(&sorted[k]), s, a, novl);
-  }
-  const int NR = R + R * (2 * R + 1);
-  for (int r = 0; r < NR; ++r) {
-    int y, z;
-    if (r < R) {
-      y = c.y + 1 + r;
-      z = c.z;
-    } else {
-      int q = r - R;
-      y = c.y - R + q % (2 * R + 1);
-      z = c.z + 1 + q / (2 * R + 1);
+  const int rows = FULL ? W * W : 1 + R + R * W;
+  for (int r = sub; r < rows; r += L) {
+    int y = c.y + r, z = c.z;
+    if (FULL) {
+      y = c.y - R + r % W;
+      z = c.z - R + r / W;
+    } else if (r > R) {
+      y = c.y - R + (r - 1 - R) % W;
+      z = c.z + 1 + (r - 1 - R) / W;
     }
-    if (y < 0 || y >= cps || z >= cps) continue;
-    int row = g0 + (z * cps + y) * cps;
-    for (uint32_t k = __ldg(&start[row + x0]), e = __ldg(&start[row + x1 + 1]); k < e; ++k)
+    if (y < 0 || y >= cps || z < 0 || z >= cps) continue;
+    const int row = g0 + (z * cps + y) * cps;
+    const uint32_t b = (!FULL && r == 0) ? (uint32_t)slot + 1u : __ldg(&start[row + x0]);
+    for (uint32_t k = b, e = __ldg(&start[row + x1 + 1]); k < e; ++k)
       contact_pair(p, bi, __ldg(&sorted[k]), s, a, novl);
   }
 }
@@ -1490,9 +1476,12 @@ __device__ __forceinline__ void contact_rows(float4 p, const ContactBead &bi, in
 // Every unordered pair is visited once, over half stencils: one grid, or the
 // typed layout's A-A half, A-other full and other-other half stencils (the
 // contact predicate is symmetric in i and j). REACH as for the pair kernel
-// (cells of side >= cutoff / REACH); 0: each system's own reach.
-template <int REACH = 1>
-__global__ void __launch_bounds__(256)
+// (cells of side >= cutoff / REACH); 0: each system's own reach. L lanes share
+// a bead's rows (blocks of tile * L threads): a thread a bead left a batch of
+// 2048 beads on 32 CTAs for 110 us, eight lanes take 21; 30386 beads (four) 37 and
+// 18 us, 131072 (two) 113 and 77.
+template <int REACH, int L>
+__global__ void __launch_bounds__(L == 1 ? 256 : 512, L == 1 ? 5 : 2)
     k_contacts_half(const Tile *__restrict__ tiles, const SysDesc *__restrict__ sys,
                     const float4 *__restrict__ sorted, const uint32_t *__restrict__ start,
                     ContactArgs a) {
@@ -1500,7 +1489,7 @@ __global__ void __launch_bounds__(256)
   pdl_trigger();
   Tile t = tiles[blockIdx.x];
   const SysDesc &s = sys[t.sys];
-  int slot = t.begin + threadIdx.x;
+  const int slot = t.begin + (int)threadIdx.x / L, sub = threadIdx.x % L;
   unsigned long long novl = 0;
   if (slot < s.bead_off + s.n) {
     float4 p = sorted[slot];
@@ -1509,14 +1498,12 @@ __global__ void __launch_bounds__(256)
     bool esc = false;
     CellXYZ c = cell_of(p, s, esc);
     const int R = (REACH > 0) ? REACH : s.reach;
-    if (s.cls_cells == 0) {
-      contact_rows<false>(p, bi, slot, c, s.cell_off, R, s, sorted, start, a, novl);
-    } else if (wbits(p) & BF_HET) {
-      contact_rows<false>(p, bi, slot, c, s.cell_off, R, s, sorted, start, a, novl);
-      contact_rows<true>(p, bi, slot, c, s.cell_off + s.cls_cells, R, s, sorted, start, a, novl);
-    } else {
-      contact_rows<false>(p, bi, slot, c, s.cell_off + s.cls_cells, R, s, sorted, start, a, novl);
-    }
+    const bool het = s.cls_cells == 0 || (wbits(p) & BF_HET);
+    const int g0 = het ? s.cell_off : s.cell_off + s.cls_cells;
+    contact_rows<false, L>(p, bi, slot, sub, c, g0, R, s, sorted, start, a, novl);
+    if (s.cls_cells != 0 && het)
+      contact_rows<true, L>(p, bi, slot, sub, c, s.cell_off + s.cls_cells, R, s, sorted, start, a,
+                            novl);
   }
   if (a.do_overlap) {
 #pragma unroll
@@ -1654,25 +1641,59 @@ __global__ void __launch_bounds__(256)
 
 // Mean spatial distance by separation (the sd part of calc_sd_cp,
 // chrana.cu:13-45): ds[chain_ps_off + s] += sum_p |r_{p+s} - r_p| over a chunk
-// of p, FP32 distances accumulated in FP64.
+// of p, FP32 distances accumulated in FP64. One launch for all chains, a CTA for
+// 128 separations and 256 p of one of them (CTAs tile_off[c] .. of chain c, found
+// by bisection), its positions in shared memory. A launch per chain left most
+// SMs idle: ccp's 12 chains of 2084-3170 beads took 12 x 40 us, bound by the
+// latency of one CTA's loop; together 37 us, bound by the square roots.
 constexpr int SDIST_PCHUNK = 256;
+constexpr int SDIST_SEPS = 128;
 
-__global__ void __launch_bounds__(256)
+__host__ __device__ inline long long sdist_tiles(int len, int smax) {
+  return (long long)((smax + SDIST_SEPS - 1) / SDIST_SEPS) * ((len + SDIST_PCHUNK - 1) / SDIST_PCHUNK);
+}
+
+__global__ void __launch_bounds__(SDIST_SEPS)
     k_sdist(const float4 *__restrict__ pos, const int32_t *__restrict__ chain_first,
             const int32_t *__restrict__ chain_len, const int32_t *__restrict__ chain_ps_off,
-            const int32_t *__restrict__ chain_smax, int chain, double *__restrict__ ds) {
-  int first = chain_first[chain], L = chain_len[chain], smax = chain_smax[chain];
-  int sep = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  int p0 = blockIdx.y * SDIST_PCHUNK;
+            const int32_t *__restrict__ chain_smax, const long long *__restrict__ tile_off,
+            int n_chains, long long tile0, double *__restrict__ ds) {
+  __shared__ float4 near[SDIST_PCHUNK];
+  __shared__ float far[3][SDIST_PCHUNK + SDIST_SEPS];
+  const long long t = tile0 + blockIdx.x;
+  int lo = 0, hi = n_chains;  // chain of this CTA: tile_off[lo] <= t < tile_off[lo + 1]
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (tile_off[m] <= t) lo = m;
+    else hi = m;
+  }
+  const int first = chain_first[lo], L = chain_len[lo], smax = chain_smax[lo];
+  const int nsep = (smax + SDIST_SEPS - 1) / SDIST_SEPS;
+  const int k = (int)(t - tile_off[lo]);
+  const int s0 = (k % nsep) * SDIST_SEPS + 1, p0 = (k / nsep) * SDIST_PCHUNK;
+  if (p0 >= L - s0) return;  // the whole CTA: no pair at its smallest separation
+  for (int i = threadIdx.x; i < SDIST_PCHUNK; i += SDIST_SEPS)
+    if (p0 + i < L) near[i] = pos[first + p0 + i];
+  for (int i = threadIdx.x; i < SDIST_PCHUNK + SDIST_SEPS; i += SDIST_SEPS)
+    if (p0 + s0 + i < L) {
+      const float4 q = pos[first + p0 + s0 + i];
+      far[0][i] = q.x;
+      far[1][i] = q.y;
+      far[2][i] = q.z;
+    }
+  __syncthreads();
+  const int sep = s0 + threadIdx.x;
   if (sep > smax || p0 >= L - sep) return;
-  int p1 = min(p0 + SDIST_PCHUNK, L - sep);
+  const int n = min(SDIST_PCHUNK, L - sep - p0);
   float acc = 0.0f;
-  for (int p = p0; p < p1; ++p) {
-    float4 a = pos[first + p], b = pos[first + p + sep];
-    float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) {
+    const float4 a = near[i];
+    const int j = i + threadIdx.x;
+    const float dx = far[0][j] - a.x, dy = far[1][j] - a.y, dz = far[2][j] - a.z;
     acc += sqrtf(dx * dx + dy * dy + dz * dz);
   }
-  atomicAdd(&ds[chain_ps_off[chain] + sep], (double)acc);
+  atomicAdd(&ds[chain_ps_off[lo] + sep], (double)acc);
 }
 
 // Sets the device step counter (the first scan of the next step bumps it).
