@@ -2229,6 +2229,7 @@ int ccpgpu_contact_counts(ccpgpu_sim *h, int32_t sys, int32_t *tri, size_t n) {
     const SysDesc &d = sys_of(h, sys);
     size_t m = (size_t)d.nbins * (d.nbins + 1) / 2;
     need(n >= m, "buffer too small");
+    fault_in(tri, sizeof(int32_t) * m);
     CK(cudaStreamSynchronize(e.stream));
     CK(cudaMemcpy(tri, e.map.p + d.map_off, sizeof(int32_t) * m, cudaMemcpyDeviceToHost));
   });

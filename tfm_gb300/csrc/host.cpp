@@ -2,6 +2,9 @@
 // initial-condition generator and ccp file formats.
 #include "host.h"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -9,6 +12,7 @@
 #include <iomanip>
 #include <limits>
 #include <sstream>
+#include <thread>
 #include <unordered_map>
 
 namespace ccpgpu {
@@ -507,6 +511,39 @@ bool parse_lbs_txt(const std::string &text, int n_l, std::vector<float> &xyz) {
   }
   is >> aux >> aux >> aux;
   return !is.fail();
+}
+
+// ------------------------------------------------------------ output buffers
+
+// GB300 hosts: 8.4 MB from the device into resident pageable memory take 0.06 ms
+// (as into page-locked memory), into fresh 64 KB pages 4.6 ms; 29 MB 0.17 and
+// 17 ms. Touching the missing pages here, several threads at once, takes a
+// fraction of that, and telling that none is missing a few microseconds.
+void fault_in(void *dst, size_t bytes) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  if (bytes < 4 * page) return;
+  char *const lo = static_cast<char *>(dst), *const hi = lo + bytes;
+  char *const base = lo - (reinterpret_cast<uintptr_t>(lo) % page);
+  const size_t n = (size_t)(hi - base + page - 1) / page;
+  std::vector<unsigned char> in(n, 0);
+  if (mincore(base, n * page, in.data()) != 0) return;  // not this kind of memory
+  std::vector<char *> missing;
+  for (size_t k = 0; k < n; ++k)
+    if (!(in[k] & 1)) missing.push_back(std::max(lo, base + k * page));
+  const size_t nt = std::min<size_t>(8, (missing.size() + 31) / 32);
+  auto touch = [&](size_t t) {
+    for (size_t k = t; k < missing.size(); k += nt) *static_cast<volatile char *>(missing[k]) = 0;
+  };
+  std::vector<std::thread> th;
+  for (size_t t = 1; t < nt; ++t) {
+    try {
+      th.emplace_back(touch, t);
+    } catch (const std::exception &) {  // no thread to be had: the copy faults those pages in
+      break;
+    }
+  }
+  if (nt) touch(0);
+  for (auto &t : th) t.join();
 }
 
 }  // namespace ccpgpu

@@ -159,4 +159,9 @@ inline uint32_t type_to_flags(int32_t pt, int preset) {
   return f;
 }
 
+// Makes the pages of an output buffer resident before the device writes it: a
+// copy into pages that have never been touched faults them in one by one from
+// the device's side.
+void fault_in(void *dst, size_t bytes);
+
 }  // namespace ccpgpu
