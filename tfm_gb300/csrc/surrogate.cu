@@ -154,6 +154,25 @@ struct Launcher {
   int *err = nullptr;
   long long kernels = 0;
 
+  // Launches a kernel that calls pdl_wait as a programmatic dependent of the one
+  // before: its CTAs start as that one's leave room and wait for its end, a
+  // convolution's with the weights loaded.
+  template <typename... P, typename... A>
+  void dependent(void (*kernel)(P...), dim3 grid, unsigned block, uint32_t smem, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    SCK(cudaLaunchKernelEx(&c, kernel, P(args)...));
+    ++kernels;
+  }
+
   // k_conv_tc over images of B x H x W pixels, cin -> N channels. The taps
   // must form an R x C grid with uniform steps (t = r C + c at ((r - R/2)
   // step_h, (c - C/2) step_w)), R in {1, 3}, C in {1, 3, 5}.
@@ -201,7 +220,7 @@ struct Launcher {
                                d.max_smem));                                                   \
       attr = true;                                                                             \
     }                                                                                          \
-    k_conv_tc<N_, R_, C_, CB_><<<grid, CONV_THREADS, smem, st>>>(x, w, sh, epi, err);          \
+    dependent(k_conv_tc<N_, R_, C_, CB_>, dim3((unsigned)grid), CONV_THREADS, smem, x, w, sh, epi, err); \
     launched = true;                                                                           \
   }
 #define SUR_CONV_N(R_, C_, CB_) SUR_CONV(64, R_, C_, CB_) SUR_CONV(128, R_, C_, CB_)
@@ -211,8 +230,6 @@ struct Launcher {
 #undef SUR_CONV_N
 #undef SUR_CONV
     if (!launched) throw Error(ST_ARG, "convolution configuration not instantiated");
-    SCK(cudaGetLastError());
-    ++kernels;
   }
 
   // The 3x3, 64 -> 64 channel case of conv, every input row read once. The
@@ -232,22 +249,8 @@ struct Launcher {
     const int kind = epi.out_f32 ? ROWS_GRADIENT : ROWS_FORWARD, grid = std::min(sh.total, d.sms);
     const uint32_t smem = rows_smem_bytes(kind);
     if ((int)smem > d.max_smem) throw Error(ST_ARG, "convolution weights do not fit in shared memory");
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3((unsigned)grid);
-    c.blockDim = dim3(ROWS_THREADS);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    if (kind == ROWS_GRADIENT)
-      SCK(cudaLaunchKernelEx(&c, k_conv_rows<ROWS_GRADIENT>, x, w, sh, epi, err));
-    else
-      SCK(cudaLaunchKernelEx(&c, k_conv_rows<ROWS_FORWARD>, x, w, sh, epi, err));
-    SCK(cudaGetLastError());
-    ++kernels;
+    dependent(kind == ROWS_GRADIENT ? k_conv_rows<ROWS_GRADIENT> : k_conv_rows<ROWS_FORWARD>,
+              dim3((unsigned)grid), ROWS_THREADS, smem, x, w, sh, epi, err);
   }
 
   // Weight and bias gradients: dw [taps][N][cin], db [N] (may be null).
@@ -682,6 +685,8 @@ struct Net {
   // Forward over n sequences (types/lad device arrays, rows optional) into y;
   // `training` keeps what the backward pass needs (ReLU masks, last output).
   void forward(const uint8_t *types, const uint8_t *lad, const int32_t *rows, int n, bool training) {
+    const long long P = (long long)n * M * M;
+    SCK(cudaMemsetAsync(y.p, 0, sizeof(float) * P, st));  // the output layer adds to it
     k_embed<<<blocks((long long)n * L), 256, 0, st>>>(types, lad, rows, L, n, x0.p);
     SCK(cudaGetLastError());
     ++run.kernels;
@@ -695,20 +700,17 @@ struct Net {
       e.mask_out = training ? emask[l + 1].p : nullptr;
       run.conv(l == 0 ? m_x0_128 : m_h_128[l], ly.map_w, n, 1, L, ly.cin, 128, ly.off, e);
     }
-    k_pool<<<blocks((long long)n * M * 128), 256, 0, st>>>(h[cfg.enc_layers].p, L, 128, f, n, hp.p);
-    SCK(cudaGetLastError());
-    ++run.kernels;
+    run.dependent(k_pool, dim3(blocks((long long)n * M * 128)), 256, 0, h[cfg.enc_layers].p, L, 128, f, n, hp.p);
     {
       ConvEpi e{};
       e.bias = params.p + proj.b_off;
       e.out = uv.p;
       run.conv(m_hp_128, proj.map_w, n, 1, M, 128, 128, proj.off, e);
     }
-    k_pair_fwd<<<dim3(M / PAIR_ROWS, n), 256, 0, st>>>(uv.p, params.p + E_off, M, z[0].p);
-    SCK(cudaGetLastError());
-    ++run.kernels;
-    const long long P = (long long)n * M * M;
-    SCK(cudaMemsetAsync(y.p, 0, sizeof(float) * P, st));
+    // runs of 32 columns, or of 8 where those leave SMs idle
+    const int cols = (M / PAIR_ROWS) * n >= 2 * dev_info().sms ? 32 : 8;
+    run.dependent(k_pair_fwd, dim3(M / PAIR_ROWS, n, std::max(1, 32 / cols * M / 256)), 256, 0, uv.p, params.p + E_off,
+                  M, cols, z[0].p);
     for (int l = 0; l < cfg.head_layers; ++l) {
       const Layer &ly = head[l];
       const bool last = l == cfg.head_layers - 1;
@@ -868,9 +870,7 @@ struct Net {
   // against 1.9 ms from a pinned slot by one host thread).
   void predict_out(int n, float *maps_host, size_t first, bool last) {
     const long long P = (long long)n * M * M;
-    k_predict_maps<<<blocks(P), 256, 0, st>>>(y.p, M, n, pred.p);
-    SCK(cudaGetLastError());
-    ++run.kernels;
+    run.dependent(k_predict_maps, dim3(blocks(P)), 256, 0, y.p, M, n, pred.p);
     if (!maps_host) return;
     float *dst = maps_host + first * (size_t)M * M;
     if (last) {
@@ -1099,9 +1099,7 @@ int ccpsur_predict_ps(ccpsur_net *h, const uint8_t *types, const uint8_t *lad, i
         SCK(cudaMemcpyAsync(n.in_lad.p, lad + (size_t)first * L, (size_t)b * L, cudaMemcpyHostToDevice, n.st));
       n.forward(n.in_types.p, lad ? n.in_lad.p : nullptr, nullptr, b, false);
       n.predict_out(b, nullptr, first, false);
-      k_ps_curve<<<b, 256, 0, n.st>>>(n.pred.p, M, n.ps_dev.p);
-      SCK(cudaGetLastError());
-      ++n.run.kernels;
+      n.run.dependent(k_ps_curve, dim3((unsigned)b), 256, 0, n.pred.p, M, n.ps_dev.p);
       SCK(cudaMemcpyAsync(ps + (size_t)first * M, n.ps_dev.p, sizeof(float) * (size_t)b * M,
                           cudaMemcpyDeviceToHost, n.st));
     }

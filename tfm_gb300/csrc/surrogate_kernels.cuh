@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const int wtiles = sh.W >> 7;
+  tc::pdl_trigger();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
       for (int t = 0; t < R * C; ++t)
         for (int cb = 0; cb < CB; ++cb)
           tc::tma_load_2d(w_base + (uint32_t)(t * CB + cb) * w_tile, &tmw, wbar, cb * 64, t * N);
+      tc::pdl_wait();  // the weights are older than the kernel before
       // windows issued so far to each MMA warp's ring
       uint32_t issued[MMA_WARPS] = {};
       int local = 0;
@@ -445,6 +447,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     const int half = (warp - 1 - MMA_WARPS) >> 2;
     const int row = q * 32 + lane;
     int local = 0;
+    tc::pdl_wait();
     for (int tile = blockIdx.x; tile < sh.n_tiles; tile += gridDim.x, ++local) {
       const int buf = local % ACC;
       const uint32_t use = (uint32_t)(local / ACC);
@@ -1336,6 +1339,8 @@ __global__ void __launch_bounds__(256)
 // 2 = LAD bead, the rest zero. idx (optional) selects dataset rows.
 __global__ void k_embed(const uint8_t *__restrict__ types, const uint8_t *__restrict__ lad,
                         const int32_t *__restrict__ idx, int L, int n, bf16 *__restrict__ x0) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= (long long)n * L) return;
   const int b = (int)(k / L), l = (int)(k - (long long)b * L);
@@ -1354,6 +1359,8 @@ __global__ void k_embed(const uint8_t *__restrict__ types, const uint8_t *__rest
 
 // Mean over `f` consecutive positions: h [n][L][C] -> hp [n][L / f][C].
 __global__ void k_pool(const bf16 *__restrict__ h, int L, int C, int f, int n, bf16 *__restrict__ hp) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int M = L / f;
   if (k >= (long long)n * M * C) return;
@@ -1367,13 +1374,16 @@ __global__ void k_pool(const bf16 *__restrict__ h, int L, int C, int f, int n, b
 
 // Pair features of the head input: z0[b][i][j][c] = u_i[c] v_j[c] + u_j[c] v_i[c]
 // + E[|i - j|][c], u = uv[..][0, 64), v = uv[..][64, 128). Block: PAIR_ROWS
-// consecutive rows i0.. of sample b; each warp walks runs of 32 consecutive
+// consecutive rows i0.. of sample b; each warp walks runs of `cols` consecutive
 // columns j, lane l holding channels 2l, 2l + 1 (one warp store covers a
 // pixel's 64 channels). A lane keeps u_i, v_i of the block's rows and the
 // distance embedding of every row in registers: the value row r needs at
 // column j + 1, E[|i0 + r - j - 1|], is the one row r - 1 used at column j,
 // so the window shifts by one row per column and only E[|i0 - j - 1|] is
 // loaded. Per pixel and row: u_j, v_j and one E value per PAIR_ROWS outputs.
+// A batch too small to fill the GPU takes shorter runs over more blocks
+// (gridDim.z): one map of 256^2 took 15 us as 32 blocks with runs of 32 columns,
+// PAIR_NOW with 8.
 constexpr int PAIR_ROWS = 8;
 
 __device__ __forceinline__ float2 ld_bf16x2(const bf16 *p) {
@@ -1381,7 +1391,10 @@ __device__ __forceinline__ float2 ld_bf16x2(const bf16 *p) {
 }
 
 __global__ void __launch_bounds__(256)
-    k_pair_fwd(const bf16 *__restrict__ uv, const float *__restrict__ E, int M, bf16 *__restrict__ z0) {
+    k_pair_fwd(const bf16 *__restrict__ uv, const float *__restrict__ E, int M, int cols,
+               bf16 *__restrict__ z0) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const int i0 = blockIdx.x * PAIR_ROWS, b = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int c = 2 * lane;
@@ -1394,11 +1407,11 @@ __global__ void __launch_bounds__(256)
     vi[r] = ld_bf16x2(uvb + (size_t)(i0 + r) * 128 + 64 + c);
   }
   __nv_bfloat162 *zb = reinterpret_cast<__nv_bfloat162 *>(z0 + (size_t)b * M * M * 64) + lane;
-  for (int j0 = warp * 32; j0 < M; j0 += nw * 32) {
+  for (int j0 = (blockIdx.z * nw + warp) * cols; j0 < M; j0 += gridDim.z * nw * cols) {
     float2 e[PAIR_ROWS];
 #pragma unroll
     for (int r = 0; r < PAIR_ROWS; ++r) e[r] = __ldg(E2 + (size_t)abs(i0 + r - j0) * 32);
-    const int j1 = min(j0 + 32, M);
+    const int j1 = min(j0 + cols, M);
     for (int j = j0; j < j1; ++j) {
       const float2 uj = ld_bf16x2(uvb + (size_t)j * 128 + c);
       const float2 vj = ld_bf16x2(uvb + (size_t)j * 128 + 64 + c);
@@ -1423,6 +1436,8 @@ constexpr float YHAT_MAX = 0.0f;
 
 // Prediction: contact probability exp(yhat).
 __global__ void k_predict_maps(const float *__restrict__ y, int M, int n, float *__restrict__ out) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= (long long)n * M * M) return;
   const long long b = k / ((long long)M * M);
@@ -1435,6 +1450,8 @@ __global__ void k_predict_maps(const float *__restrict__ y, int M, int n, float 
 // of its diagonal s, pred[b][i][i + s] for i < M - s, summed in FP64.
 __global__ void __launch_bounds__(256)
     k_ps_curve(const float *__restrict__ pred, int M, float *__restrict__ ps) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const float *m = pred + (size_t)blockIdx.x * M * M;
   for (int s = threadIdx.x; s < M; s += blockDim.x) {
     double acc = 0.0;
