@@ -737,7 +737,8 @@ struct Net {
     SCK(cudaMemsetAsync(loss.p, 0, sizeof(double), st));
     const long long P = (long long)n * M * M;
     const int HL = cfg.head_layers;
-    k_loss_out_bwd<<<blocks(P), 256, 0, st>>>(y.p, ds_target.p, ds_sweight.p, rows, z[HL].p, hmask[HL].p,
+    // four blocks an SM, each over many pixels
+    k_loss_out_bwd<<<std::min<unsigned>(blocks(P), 4 * dev_info().sms), 256, 0, st>>>(y.p, ds_target.p, ds_sweight.p, rows, z[HL].p, hmask[HL].p,
                                               params.p + wo_off, M, n, dyb.p, hdc[0].p, grads.p + wo_off,
                                               grads.p + bo_off, loss.p);
     SCK(cudaGetLastError());
