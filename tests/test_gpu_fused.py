@@ -119,3 +119,15 @@ def test_fused_overfull_cells(engine_lib):
     d = np.abs(a.positions() - b.positions()).max(1)
     assert np.median(d) <= 1e-4 and d.max() <= 2e-2
     assert not a.error_flags()[0][[0, 2]].any()
+
+
+@pytest.mark.parametrize("preset,n", [("ccp", 65), ("ccp", 3649), ("ccp", 49153), ("baseline", 7297),
+                                      ("baseline", 45000)])
+def test_fused_forces_as_the_sorted_path(engine_lib, preset, n):
+    a, b = _pair(_text(preset, n), preset, 5)
+    _same_start(a, b)
+    fa, fb = a.forces(), b.forces()
+    # two FP32 sums over the same terms, each within 1e-5 of max(|F|, 0.1 sum of
+    # the terms, 1 kT/sigma); relaxed starts keep the terms of a bead below 2e3
+    scale = np.maximum(np.linalg.norm(fb, axis=1), 200.0)
+    assert (np.linalg.norm(fa - fb, axis=1) / scale).max() <= 2e-5

@@ -177,7 +177,7 @@ struct Engine {
   int persist_reach = 0;
   size_t persist_bytes = 0;
   DevBuf<PGrid> d_pgrid;
-  // bucket path of small batches (fused.cuh), set up by its first steps
+  // bucket path of small batches (fused.cuh)
   bool fused = false;
   int fused_lanes = 8;                 // lanes per bead
   int f_nc = 0, f_tiles = 0;           // bucket cells of all systems, CTAs
@@ -378,6 +378,7 @@ struct Engine {
     fused = !par.pair_path_given && persist_reach == 0 &&
             nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) &&
             fused_cells(nullptr) <= FUSED_MAX_CELLS;
+    setup_fused();
     CK(cudaStreamSynchronize(stream));
   }
 
@@ -398,10 +399,11 @@ struct Engine {
     return cells;
   }
 
-  // Sets the bucket path up on its first use; false: the batch steps through
-  // the sorted path (also when there is no memory left for the buckets).
-  bool setup_fused() {
-    if (!fused || d_fgrid.p) return fused;
+  // Sets the bucket path up (with the other buffers: a first call does not pay
+  // for it); the batch steps through the sorted path when there is no memory
+  // left for the buckets.
+  void setup_fused() {
+    if (!fused) return;
     std::vector<FusedGrid> g;
     f_nc = (int)fused_cells(&g);
     // More lanes per bead shorten a kernel until its CTAs (256 / lanes beads,
@@ -438,14 +440,14 @@ struct Engine {
       }
       fcnt.release();
       d_ftiles.release();
-      return fused = false;
+      fused = false;
+      return;
     }
     CK(cudaMemcpyAsync(d_ftiles.p, tl.data(), sizeof(Tile) * tl.size(), cudaMemcpyHostToDevice,
                        stream));
     CK(cudaMemcpyAsync(d_fgrid.p, g.data(), sizeof(FusedGrid) * g.size(), cudaMemcpyHostToDevice,
                        stream));
     CK(cudaStreamSynchronize(stream));
-    return true;
   }
 
   // Fills the buckets with the current positions.
@@ -471,10 +473,12 @@ struct Engine {
     a.er = er.p;
     a.fbuf = fbuf.p;
     a.rnb = rnb.p;
-    a.slots_in = fslots[STAGE - 1].p;
-    a.slots_out = fslots[2 - STAGE].p;
-    a.ovf_in = fovf[STAGE - 1].p;
-    a.ovf_out = fovf[2 - STAGE].p;
+    a.force = xyz_stage.p;
+    constexpr int in = STAGE == 2 ? 1 : 0;
+    a.slots_in = fslots[in].p;
+    a.slots_out = fslots[1 - in].p;
+    a.ovf_in = fovf[in].p;
+    a.ovf_out = fovf[1 - in].p;
     const size_t stride = (size_t)f_nc + 1;
     a.cnt_in = fcnt.p + stride * (phase % 3);
     a.cnt_out = fcnt.p + stride * ((phase + 1) % 3);
@@ -1278,7 +1282,7 @@ struct Engine {
     }
     set_device_step();
     if (n == 0) return;
-    const bool buckets = mode == MODE_DST && setup_fused();
+    const bool buckets = fused && mode == MODE_DST;
     if (buckets) {
       build_buckets();
       hist_valid = false;
@@ -1495,19 +1499,22 @@ struct Engine {
     return o;
   }
 
-  std::vector<float> forces() {
+  // Total force at the current positions, packed, into f (3 nb floats).
+  void forces(float *f) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
-    sort_now();
-    launch_pair<MODE_DST>();
-    k_total_force<MODE_DST><<<(unsigned)htiles.size(), tile, 0, stream>>>(
-        d_tiles.p, d_sys.p, ff, pos.p, fs.p, rank.p, lbs_sorted.p, lbs_start.p, fout.p);
-    CK(cudaGetLastError());
-    k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
-    std::vector<float> f((size_t)3 * nb);
-    CK(cudaMemcpyAsync(f.data(), xyz_stage.p, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost,
-                       stream));
+    if (fused) {
+      build_buckets();
+      launch_fused<0>(fphase, false);
+    } else {
+      sort_now();
+      launch_pair<MODE_DST>();
+      k_total_force<MODE_DST><<<(unsigned)htiles.size(), tile, 0, stream>>>(
+          d_tiles.p, d_sys.p, ff, pos.p, fs.p, rank.p, lbs_sorted.p, lbs_start.p, fout.p);
+      k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
+      CK(cudaGetLastError());
+    }
+    CK(cudaMemcpyAsync(f, xyz_stage.p, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, stream));
     sync_and_check();
-    return f;
   }
 
   // -------------------------------------------------------------- init
@@ -2022,8 +2029,7 @@ int ccpgpu_compute_forces(ccpgpu_sim *h, float *f, size_t n) {
     need(h && f, "null argument");
     Engine &e = *h->e;
     need(n >= (size_t)3 * e.nb, "buffer too small");
-    auto v = e.forces();
-    std::memcpy(f, v.data(), sizeof(float) * 3 * e.nb);
+    e.forces(f);
   });
 }
 

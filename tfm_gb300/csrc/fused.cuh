@@ -54,6 +54,7 @@ struct FusedArgs {
   const SysDesc *sys;
   const FusedGrid *grid;
   float4 *pos, *er, *fbuf, *rnb;
+  float *force;  // STAGE 0
   const float4 *slots_in;
   float4 *slots_out;
   const uint32_t *cnt_in;  // per cell; [n_cells]: length of the overflow list
@@ -181,7 +182,10 @@ __device__ __forceinline__ float3 fused_lbs(float4 x, const SysDesc &s, const Fo
 }
 
 // One Heun stage (see k_update): STAGE 1 reads pos and writes er, STAGE 2
-// reads er and writes pos. S lanes read the first S slots of a cell together
+// reads er and writes pos. STAGE 0 writes the total force at pos (k_total_force)
+// as packed xyz triples: forces of 2048 ccp beads take this kernel and the
+// filling of the buckets, 12 us on the device, instead of the sort's four kernels,
+// the pair pass, the total and the packing, 33 us. S lanes read the first S slots of a cell together
 // and G cells are read at once by the S G lanes of a bead. Every lane notes
 // its hits in a bit mask (one bit per cell visited) and evaluates them
 // afterwards: few candidates are within the cutoff, and evaluated in place
@@ -202,10 +206,10 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
   __syncthreads();
   pdl_wait();
   pdl_trigger();
-  const float4 *X = (STAGE == 1) ? a.pos : a.er;
-  for (int c = blockIdx.x * THREADS + threadIdx.x; c <= a.n_cells;
-       c += gridDim.x * THREADS)
-    a.cnt_zero[c] = 0u;
+  const float4 *X = (STAGE == 2) ? a.er : a.pos;
+  if (STAGE != 0)
+    for (int c = blockIdx.x * THREADS + threadIdx.x; c <= a.n_cells; c += gridDim.x * THREADS)
+      a.cnt_zero[c] = 0u;
 
   float4 xi, r0, f1;
   float3 F;
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
   } else if (bo >= OWN) {
     // the noise warp: stage 1 draws, stage 2 takes what stage 1 drew
     const int in = io - OWN;
-    if (bo - OWN < B && in < end) {
+    if (STAGE != 0 && bo - OWN < B && in < end) {
       float3 z = make_float3(0.0f, 0.0f, 0.0f);
       if (ff.sd > 0.0f) {
         if (STAGE == 1) {
@@ -329,10 +333,18 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
   }
   __syncthreads();
   if (!mine) return;
-  const float4 fp = fpair[bo], rn = fnoise[bo];
+  const float4 fp = fpair[bo];
   F.x += fp.x;
   F.y += fp.y;
   F.z += fp.z;
+  if (STAGE == 0) {
+    float *f = a.force + 3 * (size_t)io;
+    f[0] = F.x;
+    f[1] = F.y;
+    f[2] = F.z;
+    return;
+  }
+  const float4 rn = fnoise[bo];
   float4 out;
   if (STAGE == 1) {
     float3 D = make_float3(F.x * ff.dt, F.y * ff.dt, F.z * ff.dt);
