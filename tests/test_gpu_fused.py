@@ -131,3 +131,58 @@ def test_fused_forces_as_the_sorted_path(engine_lib, preset, n):
     # the terms, 1 kT/sigma); relaxed starts keep the terms of a bead below 2e3
     scale = np.maximum(np.linalg.norm(fb, axis=1), 200.0)
     assert (np.linalg.norm(fa - fb, axis=1) / scale).max() <= 2e-5
+
+
+def _status(call):
+    from tfm_gb300.ccpgpu import CcpError
+
+    try:
+        call()
+    except CcpError as e:
+        return e.code, str(e)
+    return 0, ""
+
+
+# The sort's cells count up to 255 beads (of a class, in the baseline field's
+# two grids); more are refused, by either path.
+@pytest.mark.parametrize("preset,m,mixed,refused", [("ccp", 255, False, False), ("ccp", 256, False, True),
+                                                    ("ccp", 256, True, True), ("baseline", 255, False, False),
+                                                    ("baseline", 256, False, True),
+                                                    ("baseline", 288, True, False)])
+def test_fused_refuses_what_the_sort_refuses(engine_lib, preset, m, mixed, refused):
+    from tfm_gb300.ccpgpu import ChrSim
+
+    n = 600
+    a = ChrSim(_text(preset, n), seed=3)
+    b = ChrSim(_text(preset, n) + SORTED[preset], seed=3)
+    side = a.system_info(0).cell_side
+    k = np.arange(m)
+    x = np.zeros((n, 3), np.float32)
+    x[:m] = side * (0.05 + 0.9 / 7 * np.stack([k % 7, k // 7 % 7, k // 49], 1))  # inside one cell
+    k = np.arange(n - m)
+    x[m:] = -0.3 - 0.55 * np.stack([k % 7, k // 7 % 7, k // 49], 1)
+    types = np.arange(n, dtype=np.int32) % 2 if mixed else np.ones(n, np.int32)
+    for h in (a, b):
+        h.set_types(types)
+        h.set_lbs(a.lbs())
+        h.set_positions(x)
+        code, message = _status(h.forces)
+        assert (code != 0) == refused and ("cell list" in message) == refused
+        h.error_flags(clear=True)
+        if refused:
+            assert _status(lambda: h.run_steps(1))[0] == code
+
+
+@pytest.mark.parametrize("preset", ["ccp", "baseline"])
+def test_fused_escape_flag_as_the_sorted_path(engine_lib, preset):
+    a, b = _pair(_text(preset, 700), preset, 4)
+    _same_start(a, b)
+    s = b.system_info(0)
+    edge = s.cells_per_side / 2 * s.cell_side
+    x = a.positions()
+    for dx, escaped in ((-0.01, 0), (0.01, 1)):
+        x[5] = [edge + dx, 0.3, 0.2]
+        for h in (a, b):
+            h.set_positions(x)
+            _status(h.forces)
+            assert h.error_flags(clear=True)[0][1] == escaped

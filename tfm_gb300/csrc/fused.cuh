@@ -75,11 +75,14 @@ __device__ __forceinline__ int fused_cell(float4 p, const FusedGrid &g, bool &es
   return g.cell_off + ((z + 1) * g.cps + y + 1) * g.cps + x + 1;
 }
 
-// Inserts bead i at p (flags in w) into its cell's bucket.
-__device__ __forceinline__ void fused_insert(float4 p, int i, const FusedGrid &g, uint32_t *cnt,
-                                             float4 *slots, float4 *ovf, int n_cells, int *err) {
-  bool esc = false;
-  const int c = fused_cell(p, g, esc);
+// Inserts bead i at p (flags in w) into its cell's bucket. A bead has escaped
+// where the sort would clamp it: outside the system's sort grid.
+__device__ __forceinline__ void fused_insert(float4 p, int i, const SysDesc &s, const FusedGrid &g,
+                                             uint32_t *cnt, float4 *slots, float4 *ovf, int n_cells,
+                                             int *err) {
+  bool esc = false, clamped = false;
+  const int c = fused_cell(p, g, clamped);
+  cell_of(p, s, esc);
   if (esc) set_err(err, ERR_ESCAPE);
   const float4 q = make_float4(p.x, p.y, p.z,
                                __uint_as_float(((uint32_t)i << BF_BITS) | (wbits(p) & 7u)));
@@ -99,7 +102,7 @@ __global__ void k_fused_build(const Tile *__restrict__ tiles, const SysDesc *__r
   const SysDesc &s = sys[t.sys];
   const int i = t.begin + threadIdx.x;
   if ((int)threadIdx.x >= tile || i >= s.bead_off + s.n) return;
-  fused_insert(pos[i], i, grid[t.sys], cnt, slots, ovf, n_cells, err);
+  fused_insert(pos[i], i, s, grid[t.sys], cnt, slots, ovf, n_cells, err);
 }
 
 // Whether the pair of the bead at p (word wi, `near` = (index - 1) << 3) and
@@ -133,6 +136,13 @@ __device__ __forceinline__ void fused_test_add(float4 p, uint32_t wi, uint32_t n
     fused_add<POT, false>(p, q, ff, acc);
   else
     fused_add<POT, true>(p, q, ff, acc);
+}
+
+// Warp mask of the L lanes that share the calling lane's bead.
+template <int L>
+__device__ __forceinline__ uint32_t fused_lanes() {
+  const uint32_t lane = threadIdx.x & 31u;
+  return (uint32_t)(((1ull << L) - 1ull) << (lane & ~(uint32_t)(L - 1)));
 }
 
 // Offset of cell `it` (0 .. 26) of the stencil from its centre.
@@ -277,12 +287,26 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
                             ff, acc);
     }
     if (n_ovf && valid) {
+      uint32_t mates = 0;
       for (uint32_t k = sub; k < n_ovf; k += L) {
         const float4 q = a.ovf_in[k];
         const int gj = (int)(wbits(q) >> BF_BITS);
-        if (gj >= s.bead_off && gj < end)
+        if (gj >= s.bead_off && gj < end) {
           fused_test_add<POT>(p, wi, near, q, rc2_att, rc2_rep, ff, acc);
+          mates += bead_cell(q, s, esc) == bead_cell(p, s, esc);
+        }
       }
+      // more beads in the bead's cell of the sort than its byte counts hold
+      // (cell_add): the state is refused here too
+      for (int it = 0; it < 27; ++it) {
+        const uint32_t n = min(cnt[off[it]], (uint32_t)FUSED_CAP);
+        for (uint32_t k = sub; k < n; k += L)
+          mates += bead_cell(slots[(ptrdiff_t)off[it] * FUSED_CAP + k - ss], s, esc) == bead_cell(p, s, esc);
+      }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1)
+        mates += __shfl_xor_sync(fused_lanes<L>(), mates, o);
+      if (mates > 255u) set_err(a.err, ERR_SLOT);
     }
     if ((wi & BF_LAD) && valid && s.n_lbs > 0) {
       const float3 fl3 = fused_lbs(p, s, ff, a.lbs, a.lbs_start, sub, L);
@@ -360,8 +384,14 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
     a.pos[io] = out;
     if (blockIdx.x == 0 && bo == 0) *a.step += 1ull;
   }
-  if (!(isfinite(out.x) && isfinite(out.y) && isfinite(out.z))) set_err(a.err, ERR_NAN);
-  fused_insert(out, io, g, a.cnt_out, a.slots_out, a.ovf_out, a.n_cells, a.err);
+  if (!(isfinite(out.x) && isfinite(out.y) && isfinite(out.z))) {
+    // within no bead's cutoff, so left out: a state that is lost as a whole
+    // would otherwise fill the overflow list
+    set_err(a.err, ERR_NAN);
+    set_err(a.err, ERR_ESCAPE);
+    return;
+  }
+  fused_insert(out, io, s, g, a.cnt_out, a.slots_out, a.ovf_out, a.n_cells, a.err);
 }
 
 }  // namespace ccpgpu
