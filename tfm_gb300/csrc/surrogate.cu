@@ -767,11 +767,10 @@ struct Net {
       kc ^= 1;
     }
     const int k = kz;  // dz0
-    k_pair_bwd<<<dim3(M, n), 256, 0, st>>>(hdz[k].p, uv.p, M, duv.p);
-    k_dist_bwd<<<dim3(M, n), 256, 0, st>>>(hdz[k].p, M, dist_part.p);
+    k_pair_bwd<<<dim3(2 * M / PAIR_BWD_ROWS, n), 256, 0, st>>>(hdz[k].p, uv.p, M, duv.p, dist_part.p);
     k_dist_reduce<<<blocks((long long)M * 64), 256, 0, st>>>(dist_part.p, M, n, grads.p + E_off);
     SCK(cudaGetLastError());
-    run.kernels += 3;
+    run.kernels += 2;
     run.wgrad(m_hp_64, m_hp_128, m_duv_64, n, 1, M, 128, 128, proj.off, partial.p, partial.n, grads.p + proj.w_off,
               grads.p + proj.b_off);
     {

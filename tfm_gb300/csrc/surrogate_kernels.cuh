@@ -1568,52 +1568,76 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Gradient of the pair features w.r.t. u and v: with S_ij = dz_ij + dz_ji,
-// du_i = sum_j S_ij v_j and dv_i = sum_j S_ij u_j (per channel). Block: row i
-// of sample b; 256 threads = 4 groups over j x 64 channels. Output BF16.
-__global__ void __launch_bounds__(256)
-    k_pair_bwd(const float *__restrict__ dz, const bf16 *__restrict__ uv, int M, bf16 *__restrict__ duv) {
-  const int i = blockIdx.x, b = blockIdx.y;
-  const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const size_t MM = (size_t)M * M;
-  const float *dzb = dz + (size_t)b * MM * 64;
-  const bf16 *uvb = uv + (size_t)b * M * 128;
-  float du = 0.0f, dv = 0.0f;
-  for (int j = g; j < M; j += 4) {
-    const float s = dzb[((size_t)i * M + j) * 64 + c] + dzb[((size_t)j * M + i) * 64 + c];
-    du = fmaf(s, __bfloat162float(uvb[(size_t)j * 128 + 64 + c]), du);
-    dv = fmaf(s, __bfloat162float(uvb[(size_t)j * 128 + c]), dv);
-  }
-  __shared__ float su[4][64], sv[4][64];
-  su[g][c] = du;
-  sv[g][c] = dv;
-  __syncthreads();
-  if (g == 0) {
-    const float a = su[0][c] + su[1][c] + su[2][c] + su[3][c];
-    const float d = sv[0][c] + sv[1][c] + sv[2][c] + sv[3][c];
-    duv[((size_t)b * M + i) * 128 + c] = __float2bfloat16_rn(a);
-    duv[((size_t)b * M + i) * 128 + 64 + c] = __float2bfloat16_rn(d);
-  }
+// Gradients of the pair features from dz, the gradient of the head's input.
+// Blocks below M / 4 of sample b: four rows i of u and v. With S_ij = dz_ij +
+// dz_ji, du_i = sum_j S_ij v_j and dv_i = sum_j S_ij u_j per channel, output
+// BF16. The other blocks: four separations s of the distance embedding,
+// part[b][s][c] = sum over pairs with |i - j| = s of dz_ij[c] (both
+// triangles); k_dist_reduce adds the samples in order. A row or separation has
+// 64 threads: four channels each, four classes over j (over i), added in
+// order.
+//
+// dz is read three times: as dz_ij, as dz_ji and by diagonals. Blocks of both
+// kinds run side by side, sample by sample, so L2 serves two of the three, and
+// a thread reads 16 bytes at a time. Measured at 32 maps of 256^2: a kernel per
+// gradient with 4-byte loads 148 + 101 us, this one 147; HBM floor 80. L2
+// bounds it: other unrolls (2, 8, 16), fewer or more resident blocks and another order of
+// the blocks made no difference or were slower. The order of each sum (four
+// classes of j) is kept on purpose: du and dv are rounded to BF16 next, and
+// another order flips roundings (gradients of small batches then move by 8e-5).
+constexpr int PAIR_BWD_ROWS = 4;
+__device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
-
-// Gradient of the distance embedding, per sample: part[b][s][c] = sum over
-// pairs with |i - j| = s of dz_ij[c] (both triangles). Block: (s, b); 64
-// channels x 4 groups over i. k_dist_reduce adds the samples in order.
+__device__ __forceinline__ void f4_fma(float4 a, uint2 w, float4 &d) {
+  d.x = fmaf(a.x, bf_lo(w.x), d.x);
+  d.y = fmaf(a.y, bf_hi(w.x), d.y);
+  d.z = fmaf(a.z, bf_lo(w.y), d.z);
+  d.w = fmaf(a.w, bf_hi(w.y), d.w);
+}
 __global__ void __launch_bounds__(256)
-    k_dist_bwd(const float *__restrict__ dz, int M, float *__restrict__ part) {
-  const int s = blockIdx.x, b = blockIdx.y;
-  const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
+    k_pair_bwd(const float *__restrict__ dz, const bf16 *__restrict__ uv, int M, bf16 *__restrict__ duv,
+               float *__restrict__ part) {
+  const int b = blockIdx.y, row = threadIdx.x >> 6, g = (threadIdx.x >> 4) & 3, c = 4 * (threadIdx.x & 15);
   const size_t MM = (size_t)M * M;
-  const float *dzb = dz + (size_t)b * MM * 64;
-  float acc = 0.0f;
-  for (int i = g; i + s < M; i += 4) {
-    acc += dzb[((size_t)i * M + i + s) * 64 + c];
-    if (s) acc += dzb[((size_t)(i + s) * M + i) * 64 + c];
+  const float *dzb = dz + (size_t)b * MM * 64 + c;
+  const bool dist = (int)blockIdx.x >= M / PAIR_BWD_ROWS;
+  const int i = ((int)blockIdx.x - (dist ? M / PAIR_BWD_ROWS : 0)) * PAIR_BWD_ROWS + row;
+  auto at = [&](int r, int k) { return *reinterpret_cast<const float4 *>(dzb + ((size_t)r * M + k) * 64); };
+  __shared__ float4 su[4][4][16], sv[4][4][16];  // class, row, channels
+  float4 du = make_float4(0.0f, 0.0f, 0.0f, 0.0f), dv = du;
+  if (!dist) {
+    const bf16 *uvb = uv + (size_t)b * M * 128 + c;
+#pragma unroll 4
+    for (int j = g; j < M; j += 4) {
+      const float4 s = f4_add(at(i, j), at(j, i));
+      f4_fma(s, *reinterpret_cast<const uint2 *>(uvb + (size_t)j * 128 + 64), du);
+      f4_fma(s, *reinterpret_cast<const uint2 *>(uvb + (size_t)j * 128), dv);
+    }
+    sv[g][row][c / 4] = dv;
+  } else if (i) {
+#pragma unroll 4
+    for (int k = g; k < M - i; k += 4) {
+      du = f4_add(du, at(k, k + i));
+      du = f4_add(du, at(k + i, k));
+    }
+  } else {
+#pragma unroll 4
+    for (int k = g; k < M; k += 4) du = f4_add(du, at(k, k));
   }
-  __shared__ float r[4][64];
-  r[g][c] = acc;
+  su[g][row][c / 4] = du;
   __syncthreads();
-  if (g == 0) part[((size_t)b * M + s) * 64 + c] = r[0][c] + r[1][c] + r[2][c] + r[3][c];
+  if (g) return;
+  const int q = c / 4;
+  const float4 a = f4_add(f4_add(f4_add(su[0][row][q], su[1][row][q]), su[2][row][q]), su[3][row][q]);
+  if (dist) {
+    *reinterpret_cast<float4 *>(part + ((size_t)b * M + i) * 64 + c) = a;
+    return;
+  }
+  const float4 d = f4_add(f4_add(f4_add(sv[0][row][q], sv[1][row][q]), sv[2][row][q]), sv[3][row][q]);
+  bf16 *o = duv + ((size_t)b * M + i) * 128 + c;
+  *reinterpret_cast<uint2 *>(o) = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
+  *reinterpret_cast<uint2 *>(o + 64) = make_uint2(pack_bf16(d.x, d.y), pack_bf16(d.z, d.w));
 }
 
 __global__ void k_dist_reduce(const float *__restrict__ part, int M, int n, float *__restrict__ dE) {
