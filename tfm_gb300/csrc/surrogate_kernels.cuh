@@ -1026,11 +1026,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const int HW = sh.H * sh.W;
+  tc::pdl_trigger();
 
   if (warp == 0) {
     if (lane == 0) {
       tc::prefetch_map(&tmx);
       tc::prefetch_map(&tmy);
+      tc::pdl_wait();
       const uint32_t bytes = (uint32_t)(ny + nxg) * WG_TILE;
       int i = 0;
       for (; i < nkb; ++i) {
@@ -1081,6 +1083,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   } else {
     const int q = warp & 3;
     const int row = q * 32 + lane;
+    tc::pdl_wait();
     if (nkb > 0 && tc::mbar_wait(done, 0, abort)) {
       tc::fence_after_sync();
       for (int j = j0; j < j1; ++j) {
@@ -1171,11 +1174,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   const int f1 = (int)((long long)sh.total * (blockIdx.x + 1) / gridDim.x);
   RowRun run;
   int wb = 0;
+  tc::pdl_trigger();
 
   if (warp == 0) {
     if (lane == 0) {
       tc::prefetch_map(&tmx);
       tc::prefetch_map(&tmy);
+      tc::pdl_wait();
       uint32_t nx = 0, ny = 0;  // windows and gradient rows issued
       bool ok = true;
       while (ok && bands_next(sh, f, wb, f1, run)) {
@@ -1278,6 +1283,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     tc::mbar_drain(fin, 0);
   } else {
     const int row = (warp & 3) * 32 + lane;
+    tc::pdl_wait();
     if (tc::mbar_wait(done, 0, abort)) {
       tc::fence_after_sync();
       for (int p = 0; p < 2; ++p) {
@@ -1315,6 +1321,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 __global__ void __launch_bounds__(256)
     k_wgrad_reduce(const float *__restrict__ partial, int chunks, int n_atoms, int n_x, int N, int cin_blocks,
                    float *__restrict__ dw, float *__restrict__ db) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const int ci = threadIdx.x & 63, g = threadIdx.x >> 6;
   const int a = blockIdx.x / N, co = blockIdx.x - a * N;  // a == n_x: the bias row
   float s = 0.0f;
@@ -1483,6 +1491,8 @@ __global__ void __launch_bounds__(256)
                    const int32_t *__restrict__ idx, const bf16 *__restrict__ z, const uint32_t *__restrict__ mask,
                    const float *__restrict__ wo, int M, int n, float *__restrict__ dy, bf16 *__restrict__ dc,
                    float *__restrict__ gwo, float *__restrict__ gbo, double *__restrict__ loss) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = (lane & 7) * 8;
   const long long MM = (long long)M * M, P = (long long)n * MM;
@@ -1598,6 +1608,8 @@ __device__ __forceinline__ void f4_fma(float4 a, uint2 w, float4 &d) {
 __global__ void __launch_bounds__(256)
     k_pair_bwd(const float *__restrict__ dz, const bf16 *__restrict__ uv, int M, bf16 *__restrict__ duv,
                float *__restrict__ part) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const int b = blockIdx.y, row = threadIdx.x >> 6, g = (threadIdx.x >> 4) & 3, c = 4 * (threadIdx.x & 15);
   const size_t MM = (size_t)M * M;
   const float *dzb = dz + (size_t)b * MM * 64 + c;
@@ -1641,6 +1653,8 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void k_dist_reduce(const float *__restrict__ part, int M, int n, float *__restrict__ dE) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= M * 64) return;
   float s = 0.0f;
@@ -1653,6 +1667,8 @@ __global__ void k_dist_reduce(const float *__restrict__ part, int M, int n, floa
 // encoder layer's ReLU bits (BF16). C = 128.
 __global__ void k_unpool(const float *__restrict__ dhp, const uint32_t *__restrict__ mask, int L, int f,
                          int n, float *__restrict__ dz, bf16 *__restrict__ dc) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // (b, l, 16-channel chunk)
   if (k >= (long long)n * L * 8) return;
   const int c0 = (int)(k & 7) * 16;
