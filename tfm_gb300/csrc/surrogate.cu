@@ -117,6 +117,15 @@ static CUtensorMap weight_map(const void *ptr, int cin, int rows, int box_rows) 
   return m;
 }
 
+// A convolution's weights by all output channels, and by 64 of them.
+struct WeightMaps {
+  CUtensorMap all, half;
+};
+
+static WeightMaps weight_maps(const void *ptr, int cin, int taps, int cout) {
+  return {weight_map(ptr, cin, taps * cout, cout), weight_map(ptr, cin, taps * cout, 64)};
+}
+
 // ------------------------------------------------------------------ layer launchers
 
 struct DevInfo {
@@ -179,7 +188,7 @@ struct Launcher {
   // k_conv_tc over images of B x H x W pixels, cin -> N channels. The taps
   // must form an R x C grid with uniform steps (t = r C + c at ((r - R/2)
   // step_h, (c - C/2) step_w)), R in {1, 3}, C in {1, 3, 5}.
-  void conv(const CUtensorMap &x, const CUtensorMap &w, int B, int H, int W, int cin, int N, const Taps &taps,
+  void conv(const CUtensorMap &x, const WeightMaps &w, int B, int H, int W, int cin, int N, const Taps &taps,
             const ConvEpi &epi) {
     const DevInfo &d = dev_info();
     if (W % 128 || (cin != 64 && cin != 128) || (N != 64 && N != 128))
@@ -203,33 +212,41 @@ struct Launcher {
     if (std::abs(sh.step_w) * (C / 2) > WIN_RADIUS) throw Error(ST_ARG, "tap column offset above the window radius");
     const int cb = cin / 64;
     if (R == 3 && cb == 1 && N == 64 && sh.step_h != 0) {
-      conv_rows(x, w, B, H, W, sh.step_h, sh.step_w, epi);
+      conv_rows(x, w.all, B, H, W, sh.step_h, sh.step_w, epi);
       return;
     }
-    sh.stages = MAX_STAGES;
-    while (sh.stages > MMA_WARPS && (int)conv_smem_bytes(nt, cb, N, sh.stages) > d.max_smem)
-      sh.stages -= MMA_WARPS;
-    const uint32_t smem = conv_smem_bytes(nt, cb, N, sh.stages);
-    if ((int)smem > d.max_smem) throw Error(ST_ARG, "convolution weights do not fit in shared memory");
     sh.n_tiles = B * H * (W / 128);
     if (sh.n_tiles == 0) return;
-    const int grid = std::min(sh.n_tiles, d.sms);
+    // two CTAs a tile, 64 channels each, where the tiles leave SMs idle. us, whole
+    // / split: prediction of 1 map 158 / 148, 4 228 / 215, 9 (72 tiles) 344 / 334;
+    // loss and gradients of 3 maps of 128^2 588 / 545
+    const bool split = N == 128 && R == 1 && 2 * sh.n_tiles <= d.sms;
+    const int nc = split ? 64 : N;
+    sh.stages = MAX_STAGES;
+    while (sh.stages > MMA_WARPS && (int)conv_smem_bytes(nt, cb, nc, sh.stages) > d.max_smem)
+      sh.stages -= MMA_WARPS;
+    const uint32_t smem = conv_smem_bytes(nt, cb, nc, sh.stages);
+    if ((int)smem > d.max_smem) throw Error(ST_ARG, "convolution weights do not fit in shared memory");
+    const dim3 grid((unsigned)std::min(sh.n_tiles, d.sms), split ? 2u : 1u);
     bool launched = false;
-#define SUR_CONV(N_, R_, C_, CB_)                                                              \
-  if (N == N_ && R == R_ && C == C_ && cb == CB_) {                                            \
+#define SUR_CONV(N_, R_, C_, CB_, LD_)                                                         \
+  if (nc == N_ && N == LD_ && R == R_ && C == C_ && cb == CB_) {                               \
     static bool attr = false;                                                                  \
     if (!attr) {                                                                               \
-      SCK(cudaFuncSetAttribute(k_conv_tc<N_, R_, C_, CB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                               d.max_smem));                                                   \
+      SCK(cudaFuncSetAttribute(k_conv_tc<N_, R_, C_, CB_, LD_>,                                \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem));      \
       attr = true;                                                                             \
     }                                                                                          \
-    dependent(k_conv_tc<N_, R_, C_, CB_>, dim3((unsigned)grid), CONV_THREADS, smem, x, w, sh, epi, err); \
+    dependent(k_conv_tc<N_, R_, C_, CB_, LD_>, grid, CONV_THREADS, smem, x,                   \
+              split ? w.half : w.all, sh, epi, err);                                           \
     launched = true;                                                                           \
   }
-#define SUR_CONV_N(R_, C_, CB_) SUR_CONV(64, R_, C_, CB_) SUR_CONV(128, R_, C_, CB_)
+#define SUR_CONV_N(R_, C_, CB_) SUR_CONV(64, R_, C_, CB_, 64) SUR_CONV(128, R_, C_, CB_, 128)
+#define SUR_CONV_1(C_, CB_) SUR_CONV_N(1, C_, CB_) SUR_CONV(64, 1, C_, CB_, 128)
     // (64, 3, 3, 1): rows that all read the same input row; the rest is conv_rows
-    SUR_CONV_N(3, 3, 1) SUR_CONV_N(3, 3, 2) SUR_CONV_N(1, 5, 1) SUR_CONV_N(1, 5, 2)
-    SUR_CONV_N(1, 3, 1) SUR_CONV_N(1, 3, 2) SUR_CONV_N(1, 1, 1) SUR_CONV_N(1, 1, 2)
+    SUR_CONV_N(3, 3, 1) SUR_CONV_N(3, 3, 2) SUR_CONV_1(5, 1) SUR_CONV_1(5, 2)
+    SUR_CONV_1(3, 1) SUR_CONV_1(3, 2) SUR_CONV_1(1, 1) SUR_CONV_1(1, 2)
+#undef SUR_CONV_1
 #undef SUR_CONV_N
 #undef SUR_CONV
     if (!launched) throw Error(ST_ARG, "convolution configuration not instantiated");
@@ -422,7 +439,7 @@ struct Layer {
   Taps off;
   size_t w_off = 0, b_off = 0;
   Buf<bf16> wb, wt;
-  CUtensorMap map_w{}, map_wt{};
+  WeightMaps map_w{}, map_wt{};
 };
 
 struct Net {
@@ -539,8 +556,8 @@ struct Net {
     for (Layer *l : all_layers()) {
       l->wb.alloc((size_t)l->taps * l->cout * l->cin);
       l->wt.alloc((size_t)l->taps * l->cout * l->cin);
-      l->map_w = weight_map(l->wb.p, l->cin, l->taps * l->cout, l->cout);
-      l->map_wt = weight_map(l->wt.p, l->cout, l->taps * l->cin, l->cin);
+      l->map_w = weight_maps(l->wb.p, l->cin, l->taps, l->cout);
+      l->map_wt = weight_maps(l->wt.p, l->cout, l->taps, l->cin);
     }
     refresh_weights();
     alloc_activations();
@@ -1205,7 +1222,7 @@ int ccpsur_conv_bf16(int32_t B, int32_t H, int32_t W, int32_t cin, int32_t cout,
     run.st = st;
     run.err = derr.p;
     CUtensorMap mx = image_map(dx.p, cin, W, H, B, WIN_ROWS);
-    CUtensorMap mw = weight_map(dwb.p, cin, ntaps * cout, cout);
+    const WeightMaps mw = weight_maps(dwb.p, cin, ntaps, cout);
     run.conv(mx, mw, B, H, W, cin, cout, taps, e);
     int flags = 0;
     SCK(cudaMemcpyAsync(out, dout.p, P * cout * 2, cudaMemcpyDeviceToHost, st));

@@ -166,22 +166,23 @@ __device__ __forceinline__ void load_row_bf16x32(const bf16 *src, size_t pbase, 
   __syncwarp();
 }
 
-template <int N>
-__device__ __forceinline__ void conv_epilogue_load(const ConvEpi &e, size_t p, int half, EpiLoads<N> &ld,
-                                                   uint4 *stage) {
+// N: the CTA's channels, from c_base on, of the LD of a pixel.
+template <int N, int LD>
+__device__ __forceinline__ void conv_epilogue_load(const ConvEpi &e, size_t p, int c_base, int half,
+                                                   EpiLoads<N> &ld, uint4 *stage) {
   constexpr int G = N / 64;  // 32-column groups per thread
-  const int c_begin = half * (N / 2);
+  const int c_begin = c_base + half * (N / 2);
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    const size_t o = p * (size_t)N + c_begin + 32 * g;
+    const size_t o = p * (size_t)LD + c_begin + 32 * g;
     if (e.resid)
-      load_row_bf16x32<N>(e.resid, p - (size_t)(threadIdx.x & 31), c_begin + 32 * g, ld.rb[g], stage);
+      load_row_bf16x32<LD>(e.resid, p - (size_t)(threadIdx.x & 31), c_begin + 32 * g, ld.rb[g], stage);
     if (e.resid_f32) {
       const float4 *s = reinterpret_cast<const float4 *>(e.resid_f32 + o);
 #pragma unroll
       for (int i = 0; i < 8; ++i) ld.rf[g][i] = s[i];
     }
-    if (e.mask_in) ld.mi[g] = e.mask_in[p * (N / 32) + (c_begin >> 5) + g];
+    if (e.mask_in) ld.mi[g] = e.mask_in[p * (LD / 32) + (c_begin >> 5) + g];
   }
   ld.rdy = e.resid_dy ? e.resid_dy[p] : 0.0f;
 }
@@ -216,10 +217,10 @@ __device__ __forceinline__ void store_row_bf16x32(bf16 *out, size_t pbase, int c
 // (32 N / 64 columns from TMEM address taddr), with its global inputs in ld;
 // stage: the warp's 2 KB staging tile for the BF16 output.
 // Returns this thread's partial output-layer dot (0 without wo).
-template <int N>
+template <int N, int LD>
 __device__ __forceinline__ float conv_epilogue_row(const ConvEpi &e, const float *sbias, const float *swo,
-                                                   size_t p, int half, uint32_t taddr, const EpiLoads<N> &ld,
-                                                   uint4 *stage) {
+                                                   size_t p, int c_base, int half, uint32_t taddr,
+                                                   const EpiLoads<N> &ld, uint4 *stage) {
   constexpr int G = N / 64;
   const int c_begin = half * (N / 2);
   const float rdy = ld.rdy;
@@ -237,7 +238,7 @@ __device__ __forceinline__ float conv_epilogue_row(const ConvEpi &e, const float
       uint32_t bits = 0;
 #pragma unroll
       for (int i = 0; i < 32; ++i) bits |= (v[i] > 0.0f ? 1u : 0u) << i;
-      e.mask_out[p * (N / 32) + (c0 >> 5)] = bits;
+      e.mask_out[p * (LD / 32) + ((c_base + c0) >> 5)] = bits;
     }
     if (e.relu) {
 #pragma unroll
@@ -267,7 +268,7 @@ __device__ __forceinline__ float conv_epilogue_row(const ConvEpi &e, const float
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = fmaf(rdy, swo[c0 + i], v[i]);
     }
-    const size_t o = p * (size_t)N + c0;
+    const size_t o = p * (size_t)LD + c_base + c0;
     if (e.out_f32) {
       float4 *d = reinterpret_cast<float4 *>(e.out_f32 + o);
 #pragma unroll
@@ -281,16 +282,19 @@ __device__ __forceinline__ float conv_epilogue_row(const ConvEpi &e, const float
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = ((ld.mi[g] >> i) & 1u) ? v[i] : 0.0f;
     }
-    if (e.out) store_row_bf16x32<N>(e.out, p - (size_t)(threadIdx.x & 31), c0, v, stage);
+    if (e.out) store_row_bf16x32<LD>(e.out, p - (size_t)(threadIdx.x & 31), c_base + c0, v, stage);
   }
   return dot;
 }
 
 // Implicit-GEMM convolution (see the file comment). tmx: 4-D map over the
 // input image {C, W, H, B} with box {64, 128, 1, 1}; tmw: 2-D map over the
-// weights {C_in, taps x N} with box {64, N}, both with 128-byte swizzle.
-// Grid: persistent, at most one CTA per SM; tiles strided by gridDim.x.
-template <int N, int R, int C, int CB>
+// weights {C_in, taps x LD} with box {64, N}, both with 128-byte swizzle.
+// Grid: persistent, at most one CTA per SM; tiles strided by gridDim.x. A CTA
+// computes N of the LD output channels, those of blockIdx.y: with too few tiles
+// for the SMs two CTAs share a tile, which halves its weights, MMAs and
+// epilogue. A value's sum is the same either way.
+template <int N, int R, int C, int CB, int LD = N>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
     k_conv_tc(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
               const ConvShape sh, const ConvEpi epi, int *err) {
@@ -335,7 +339,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     *abort = 0;
     tc::fence_barrier_init();
   }
-  for (int k = threadIdx.x; k < N; k += blockDim.x) sbias[k] = epi.bias ? epi.bias[k] : 0.0f;
+  const int c_base = N == LD ? 0 : (int)blockIdx.y * N;
+  for (int k = threadIdx.x; k < N; k += blockDim.x) sbias[k] = epi.bias ? epi.bias[c_base + k] : 0.0f;
   for (int k = threadIdx.x; k < 64; k += blockDim.x) swo[k] = epi.wo ? epi.wo[k] : 0.0f;
   if (warp == 1) tc::tmem_alloc(tc::smem_u32(tmem_slot), TMEM_COLS_CONV);
   tc::fence_before_sync();
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
       tc::mbar_arrive_expect_tx(wbar, (uint32_t)nwt * w_tile);
       for (int t = 0; t < R * C; ++t)
         for (int cb = 0; cb < CB; ++cb)
-          tc::tma_load_2d(w_base + (uint32_t)(t * CB + cb) * w_tile, &tmw, wbar, cb * 64, t * N);
+          tc::tma_load_2d(w_base + (uint32_t)(t * CB + cb) * w_tile, &tmw, wbar, cb * 64, t * LD + c_base);
       tc::pdl_wait();  // the weights are older than the kernel before
       // windows issued so far to each MMA warp's ring
       uint32_t issued[MMA_WARPS] = {};
@@ -455,11 +460,11 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
       const size_t p = (size_t)bh * sh.W + (size_t)wb * 128 + row;
       EpiLoads<N> ld;
       uint4 *stage = epi_stage + (warp - 1 - MMA_WARPS) * (EPI_STAGE_BYTES / 16);
-      conv_epilogue_load<N>(epi, p, half, ld, stage);  // before the accumulator is ready
+      conv_epilogue_load<N, LD>(epi, p, c_base, half, ld, stage);  // before the accumulator is ready
       if (!tc::mbar_wait(tfull0 + 8u * buf, use & 1u, abort)) break;
       tc::fence_after_sync();
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * N);
-      const float dot = conv_epilogue_row<N>(epi, sbias, swo, p, half, taddr, ld, stage);
+      const float dot = conv_epilogue_row<N, LD>(epi, sbias, swo, p, c_base, half, taddr, ld, stage);
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(tempty0 + 8u * buf);
