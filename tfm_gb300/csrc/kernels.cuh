@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "sdist.h"
 
 namespace ccpgpu {
 
@@ -1646,13 +1647,6 @@ __global__ void __launch_bounds__(256)
 // by bisection), its positions in shared memory. A launch per chain left most
 // SMs idle: ccp's 12 chains of 2084-3170 beads took 12 x 40 us, bound by the
 // latency of one CTA's loop; together 37 us, bound by the square roots.
-constexpr int SDIST_PCHUNK = 256;
-constexpr int SDIST_SEPS = 128;
-
-__host__ __device__ inline long long sdist_tiles(int len, int smax) {
-  return (long long)((smax + SDIST_SEPS - 1) / SDIST_SEPS) * ((len + SDIST_PCHUNK - 1) / SDIST_PCHUNK);
-}
-
 __global__ void __launch_bounds__(SDIST_SEPS)
     k_sdist(const float4 *__restrict__ pos, const int32_t *__restrict__ chain_first,
             const int32_t *__restrict__ chain_len, const int32_t *__restrict__ chain_ps_off,
@@ -1668,9 +1662,8 @@ __global__ void __launch_bounds__(SDIST_SEPS)
     else hi = m;
   }
   const int first = chain_first[lo], L = chain_len[lo], smax = chain_smax[lo];
-  const int nsep = (smax + SDIST_SEPS - 1) / SDIST_SEPS;
-  const int k = (int)(t - tile_off[lo]);
-  const int s0 = (k % nsep) * SDIST_SEPS + 1, p0 = (k / nsep) * SDIST_PCHUNK;
+  int s0, p0;
+  sdist_tile(t - tile_off[lo], smax, s0, p0);
   if (p0 >= L - s0) return;  // the whole CTA: no pair at its smallest separation
   for (int i = threadIdx.x; i < SDIST_PCHUNK; i += SDIST_SEPS)
     if (p0 + i < L) near[i] = pos[first + p0 + i];
