@@ -140,25 +140,20 @@ constexpr float LJ_Z2_HI = 1.259921074e+00f;
 constexpr float LJ_Z2_LO = -2.401870169e-08f;
 constexpr float LJ_Z2_SQ = 1.587401032e+00f;
 
-// d^2 - (kh + kl) for the vector (dx, dy, dz) without cancellation where d^2 is
-// within a factor 2 of kh < 8: each component is split as x = xh + xl with xh on
-// a 2^-10 grid (rounded by adding and subtracting 1.5 * 2^13), so xh^2 and the
-// sum of the three are exact in FP32 and the sum minus kh is exact (Sterbenz);
-// x^2 - xh^2 = xl (xh + x) is small. Elsewhere nothing cancels.
-__device__ __forceinline__ float sq3_gap(float dx, float dy, float dz, float kh, float kl) {
+// d^2 - 2^(1/3) for the pair vector (dx, dy, dz), |components| < 2, without
+// cancellation: each component is split as x = xh + xl with xh on a 2^-10
+// grid (rounded by adding and subtracting 1.5 * 2^13), so xh^2 and the sum of
+// the three are exact in FP32 and the sum minus 2^(1/3) is exact (Sterbenz)
+// for d^2 within a factor 2 of it; x^2 - xh^2 = xl (xh + x) is small.
+__device__ __forceinline__ float lj_zero_gap(float dx, float dy, float dz) {
   const float M = 12288.0f;
   float xh = __fsub_rn(__fadd_rn(dx, M), M), yh = __fsub_rn(__fadd_rn(dy, M), M),
         zh = __fsub_rn(__fadd_rn(dz, M), M);
   float sh = __fmaf_rn(zh, zh, __fmaf_rn(yh, yh, __fmul_rn(xh, xh)));
   float lo = __fmaf_rn(__fsub_rn(dx, xh), __fadd_rn(xh, dx),
                        __fmaf_rn(__fsub_rn(dy, yh), __fadd_rn(yh, dy),
-                                 __fmaf_rn(__fsub_rn(dz, zh), __fadd_rn(zh, dz), -kl)));
-  return __fadd_rn(__fsub_rn(sh, kh), lo);
-}
-
-// d^2 - 2^(1/3), the gap to the Lennard-Jones force's zero.
-__device__ __forceinline__ float lj_zero_gap(float dx, float dy, float dz) {
-  return sq3_gap(dx, dy, dz, LJ_Z2_HI, LJ_Z2_LO);
+                                 __fmaf_rn(__fsub_rn(dz, zh), __fadd_rn(zh, dz), -LJ_Z2_LO)));
+  return __fadd_rn(__fsub_rn(sh, LJ_Z2_HI), lo);
 }
 
 // Lennard-Jones coefficient 24 e (2 / d^14 - 1 / d^8) = 24 e d^-8 (2 d^-6 - 1)
@@ -1207,14 +1202,14 @@ __device__ __forceinline__ float3 bonded_force_at(Load X, int i, float4 xi, int 
   if (e1) {
     float cx = v1.x * two_sum_err(xi.x, -xm1.x, v1.x) + v1.y * two_sum_err(xi.y, -xm1.y, v1.y) +
                v1.z * two_sum_err(xi.z, -xm1.z, v1.z);
-    float s1 = __fadd_rn(sq3_gap(v1.x, v1.y, v1.z, lh, ll), 2.0f * cx);
+    float s1 = __fadd_rn(sq3_minus(v1.x, v1.y, v1.z, lh, ll), 2.0f * cx);
     float d1 = sqrtf(v1.x * v1.x + v1.y * v1.y + v1.z * v1.z);
     ke1 = ff.k_e * (s1 / (d1 + ff.l_0)) * il1;
   }
   if (e2) {
     float cx = v2.x * two_sum_err(xp1.x, -xi.x, v2.x) + v2.y * two_sum_err(xp1.y, -xi.y, v2.y) +
                v2.z * two_sum_err(xp1.z, -xi.z, v2.z);
-    float s2 = __fadd_rn(sq3_gap(v2.x, v2.y, v2.z, lh, ll), 2.0f * cx);
+    float s2 = __fadd_rn(sq3_minus(v2.x, v2.y, v2.z, lh, ll), 2.0f * cx);
     float d2 = sqrtf(v2.x * v2.x + v2.y * v2.y + v2.z * v2.z);
     ke2 = ff.k_e * (s2 / (d2 + ff.l_0)) * il2;
   }
