@@ -1359,18 +1359,26 @@ struct Engine {
     if (e[ERR_SLOT]) throw Error(ST_STATE, "cell list inconsistent with positions");
   }
 
-  // Standalone analysis at the current positions.
+  // Standalone analysis at the current positions. Every call flags a bead that
+  // has escaped and a cell that is too full, also after the flags were cleared:
+  // the sorted path by the histogram that recount_sorted leaves for the next
+  // step, the bucket path, whose steps need none, by the one counted here.
   void sort_now() {
-    if (!hist_valid) count_cells();
+    if (fused || !hist_valid) count_cells();
     launch_scan(false);
     launch_scatter(pos.p);
     hist_valid = false;  // the scatter has used the histogram up
+  }
+
+  void recount_sorted() {
+    if (!fused) count_cells();
   }
 
   void observe(bool with_sdist) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     sort_now();
     launch_observe_sorted(with_sdist);
+    recount_sorted();
     CK(cudaGetLastError());
     ++frames_observed;
     sync_and_check();
@@ -1404,6 +1412,7 @@ struct Engine {
     k_observe<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, CCP_RCO / 2.0f, fobs.p);
     k_frame_extra<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, fextra.p);
     kcount += 2;
+    recount_sorted();
     CK(cudaGetLastError());
     ++frames_observed;
     std::vector<double> fo(ns * OBS_STRIDE), fx(ns * 2);
@@ -1491,6 +1500,7 @@ struct Engine {
     CK(cudaMemsetAsync(ovl.p, 0, sizeof(unsigned long long) * hsys.size(), stream));
     sort_now();
     launch_contacts_args(contact_args(false, false, true));
+    recount_sorted();
     CK(cudaGetLastError());
     std::vector<unsigned long long> o(hsys.size());
     CK(cudaMemcpyAsync(o.data(), ovl.p, sizeof(unsigned long long) * o.size(),
@@ -1510,6 +1520,7 @@ struct Engine {
       launch_pair<MODE_DST>();
       k_total_force<MODE_DST><<<(unsigned)htiles.size(), tile, 0, stream>>>(
           d_tiles.p, d_sys.p, ff, pos.p, fs.p, rank.p, lbs_sorted.p, lbs_start.p, fout.p);
+      recount_sorted();
       k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
       CK(cudaGetLastError());
     }
