@@ -1509,7 +1509,8 @@ struct Engine {
     return o;
   }
 
-  // Total force at the current positions, packed, into f (3 nb floats).
+  // Total force at the current positions, packed, into f (3 nb floats), which
+  // is written only when the state is not refused.
   void forces(float *f) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     if (fused) {
@@ -1524,8 +1525,9 @@ struct Engine {
       k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
       CK(cudaGetLastError());
     }
-    CK(cudaMemcpyAsync(f, xyz_stage.p, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, stream));
     sync_and_check();
+    CK(cudaMemcpyAsync(f, xyz_stage.p, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
   }
 
   // -------------------------------------------------------------- init
