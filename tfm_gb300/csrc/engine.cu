@@ -1351,34 +1351,35 @@ struct Engine {
     dev_next = ~0ull;  // the device step counter was not advanced
   }
 
-  void sync_and_check() {
+  // The device's error flags; clear also forgets the histogram and the buckets,
+  // so that the next call counts again and flags what is still wrong.
+  void read_flags(int *e, bool clear) {
     CK(cudaStreamSynchronize(stream));
+    CK(cudaMemcpy(e, d_err.p, sizeof(int) * ERR_COUNT, cudaMemcpyDeviceToHost));
+    if (!clear) return;
+    CK(cudaMemsetAsync(d_err.p, 0, sizeof(int) * ERR_COUNT, stream));
+    if (e[ERR_ESCAPE] || e[ERR_SLOT]) hist_valid = buckets_valid = false;
+  }
+
+  void sync_and_check() {
     int e[ERR_COUNT];
-    CK(cudaMemcpy(e, d_err.p, sizeof(e), cudaMemcpyDeviceToHost));
+    read_flags(e, false);
     if (e[ERR_NAN]) throw Error(ST_STATE, "non-finite bead position");
     if (e[ERR_SLOT]) throw Error(ST_STATE, "cell list inconsistent with positions");
   }
 
-  // Standalone analysis at the current positions. Every call flags a bead that
-  // has escaped and a cell that is too full, also after the flags were cleared:
-  // the sorted path by the histogram that recount_sorted leaves for the next
-  // step, the bucket path, whose steps need none, by the one counted here.
+  // Standalone analysis at the current positions.
   void sort_now() {
-    if (fused || !hist_valid) count_cells();
+    if (!hist_valid) count_cells();
     launch_scan(false);
     launch_scatter(pos.p);
     hist_valid = false;  // the scatter has used the histogram up
-  }
-
-  void recount_sorted() {
-    if (!fused) count_cells();
   }
 
   void observe(bool with_sdist) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     sort_now();
     launch_observe_sorted(with_sdist);
-    recount_sorted();
     CK(cudaGetLastError());
     ++frames_observed;
     sync_and_check();
@@ -1412,7 +1413,6 @@ struct Engine {
     k_observe<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, CCP_RCO / 2.0f, fobs.p);
     k_frame_extra<<<(unsigned)htiles.size(), tile, 0, stream>>>(d_tiles.p, d_sys.p, pos.p, fextra.p);
     kcount += 2;
-    recount_sorted();
     CK(cudaGetLastError());
     ++frames_observed;
     std::vector<double> fo(ns * OBS_STRIDE), fx(ns * 2);
@@ -1500,7 +1500,6 @@ struct Engine {
     CK(cudaMemsetAsync(ovl.p, 0, sizeof(unsigned long long) * hsys.size(), stream));
     sort_now();
     launch_contacts_args(contact_args(false, false, true));
-    recount_sorted();
     CK(cudaGetLastError());
     std::vector<unsigned long long> o(hsys.size());
     CK(cudaMemcpyAsync(o.data(), ovl.p, sizeof(unsigned long long) * o.size(),
@@ -1521,7 +1520,6 @@ struct Engine {
       launch_pair<MODE_DST>();
       k_total_force<MODE_DST><<<(unsigned)htiles.size(), tile, 0, stream>>>(
           d_tiles.p, d_sys.p, ff, pos.p, fs.p, rank.p, lbs_sorted.p, lbs_start.p, fout.p);
-      recount_sorted();
       k_pack_xyz<<<(nb + 255) / 256, 256, 0, stream>>>(fout.p, xyz_stage.p, nb);
       CK(cudaGetLastError());
     }
@@ -1968,10 +1966,7 @@ int ccpgpu_kernel_count(const ccpgpu_sim *h, uint64_t *count) {
 int ccpgpu_error_flags(ccpgpu_sim *h, int32_t *flags8, int32_t clear) {
   return guarded([&] {
     need(h && flags8, "null argument");
-    Engine &e = *h->e;
-    CK(cudaStreamSynchronize(e.stream));
-    CK(cudaMemcpy(flags8, e.d_err.p, sizeof(int) * ERR_COUNT, cudaMemcpyDeviceToHost));
-    if (clear) CK(cudaMemset(e.d_err.p, 0, sizeof(int) * ERR_COUNT));
+    h->e->read_flags(flags8, clear != 0);
     if (flags8[ERR_NAN] || flags8[ERR_SLOT]) throw Error(ST_STATE, "device error flag set");
   });
 }

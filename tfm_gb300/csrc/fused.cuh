@@ -383,9 +383,6 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
   F.y += fp.y;
   F.z += fp.z;
   if (STAGE == 0) {
-    bool esc = false;  // as the histogram of the sorted path flags it
-    cell_of(xi, s, esc);
-    if (esc) set_err(a.err, ERR_ESCAPE);
     float *f = a.force + 3 * (size_t)io;
     f[0] = F.x;
     f[1] = F.y;
