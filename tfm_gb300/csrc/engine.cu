@@ -376,17 +376,28 @@ struct Engine {
     reset_observables();
     setup_persist();
     fused = !par.pair_path_given && persist_reach == 0 &&
-            nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) &&
+            nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) && buckets_cover_sort() &&
             fused_cells(nullptr) <= FUSED_MAX_CELLS;
     setup_fused();
     CK(cudaStreamSynchronize(stream));
   }
 
-  // Bucket grids of all systems: cells of the largest pair cutoff, with a
-  // margin that keeps pairs at it within the stencil despite the rounding of
-  // the cell coordinates. Returns the number of cells.
+  // Side of the buckets: the largest pair cutoff, with a margin that keeps pairs
+  // at it within the stencil despite the rounding of the cell coordinates.
+  float bucket_side() const { return std::max(ff.rc_att, ff.rc_rep) * 1.0001f; }
+
+  // Whether the bucket path sees every cell that the sort would refuse: those
+  // no wider than a bucket (a contact cutoff beyond twice the forces' makes
+  // wider ones).
+  bool buckets_cover_sort() const {
+    for (const SysDesc &d : hsys)
+      if (!(d.csl <= bucket_side())) return false;
+    return true;
+  }
+
+  // Bucket grids of all systems. Returns the number of cells.
   int64_t fused_cells(std::vector<FusedGrid> *out) const {
-    const float csl = std::max(ff.rc_att, ff.rc_rep) * 1.0001f;
+    const float csl = bucket_side();
     int64_t cells = 0;
     for (size_t s = 0; s < hsys.size(); ++s) {
       const float half = std::ceil(geo[s].d_m / csl);
@@ -426,7 +437,7 @@ struct Engine {
     f_tiles = (int)tl.size();
     try {
       for (int k = 0; k < 2; ++k) {
-        fslots[k].alloc((size_t)f_nc * FUSED_CAP);
+        fslots[k].alloc((size_t)f_nc * FUSED_SLOTS);
         fovf[k].alloc(nb);
       }
       fcnt.alloc((size_t)3 * (f_nc + 1));
@@ -1198,7 +1209,8 @@ struct Engine {
     }
     par.pair_lanes = best_lanes;
     regrid(csl, best_tile);
-    if (had_buckets) {  // the bucket path stays where it is faster than the best of these
+    // the bucket path stays where it is faster than the best of these
+    if (had_buckets && buckets_cover_sort()) {
       fused = true;
       const double ms = time_steps(reps);
       fused = ms < best;

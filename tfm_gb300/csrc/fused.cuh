@@ -36,7 +36,12 @@
 
 namespace ccpgpu {
 
-constexpr int FUSED_CAP = 32;           // slots of a cell
+constexpr int FUSED_SLOTS = 32;         // a cell's slots in memory
+// ... of which it fills 31: a cell of the sort, which is no wider than a bucket,
+// meets at most eight buckets, so one that holds more than the 255 beads the sort
+// can count leaves some in the overflow list, where the bead's CTA looks for that.
+constexpr int FUSED_CAP = 31;
+static_assert(8 * FUSED_CAP <= 255, "an over-full cell of the sort shows as overflow");
 constexpr int FUSED_PAIR_THREADS = 256;
 // pair lanes, then a thread per bead for the other forces and one for the noise
 // (whole warps)
@@ -88,7 +93,7 @@ __device__ __forceinline__ void fused_insert(float4 p, int i, const SysDesc &s, 
                                __uint_as_float(((uint32_t)i << BF_BITS) | (wbits(p) & 7u)));
   const uint32_t r = atomicAdd(&cnt[c], 1u);
   if (r < (uint32_t)FUSED_CAP)
-    slots[(size_t)c * FUSED_CAP + r] = q;
+    slots[(size_t)c * FUSED_SLOTS + r] = q;
   else
     ovf[atomicAdd(&cnt[n_cells], 1u)] = q;
 }
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
     const int c0 = fused_cell(p, g, esc);
     const float rc2_att = ff.rc_att * ff.rc_att, rc2_rep = ff.rc_rep * ff.rc_rep;
     const uint32_t *cnt = a.cnt_in + c0;
-    const float4 *slots = a.slots_in + (size_t)c0 * FUSED_CAP + ss;
+    const float4 *slots = a.slots_in + (size_t)c0 * FUSED_SLOTS + ss;
     // one bit per cell visited: hits of A-A pairs, of other pairs, cells with
     // more than S beads
     uint32_t hit_a = 0, hit_x = 0, over = 0;
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
         // the slot is read without waiting for the count (a slot beyond it
         // holds an old position and is not a hit)
         const uint32_t n = cnt[o];
-        const float4 q = slots[(ptrdiff_t)o * FUSED_CAP];
+        const float4 q = slots[(ptrdiff_t)o * FUSED_SLOTS];
         if ((uint32_t)ss < n && fused_hit(p, wi, near, q, rc2_att, rc2_rep)) {
           if (POT == POT_LJ && !(wi & wbits(q) & BF_HET))
             hit_x |= 1u << v;
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
       if (hit_a) {
         const int o = off[(__ffs(hit_a) - 1) * G + gs];
         hit_a &= hit_a - 1u;
-        fused_add<POT, true>(p, slots[(ptrdiff_t)o * FUSED_CAP], ff, acc);
+        fused_add<POT, true>(p, slots[(ptrdiff_t)o * FUSED_SLOTS], ff, acc);
       }
     }
     if (POT == POT_LJ) {
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
         if (hit_x) {
           const int o = off[(__ffs(hit_x) - 1) * G + gs];
           hit_x &= hit_x - 1u;
-          fused_add<POT, false>(p, slots[(ptrdiff_t)o * FUSED_CAP], ff, acc);
+          fused_add<POT, false>(p, slots[(ptrdiff_t)o * FUSED_SLOTS], ff, acc);
         }
       }
     }
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
       over &= over - 1u;
       const uint32_t n = min(cnt[o], (uint32_t)FUSED_CAP);
       for (uint32_t k = S + ss; k < n; k += S)
-        fused_test_add<POT>(p, wi, near, slots[(ptrdiff_t)o * FUSED_CAP + (k - ss)], rc2_att, rc2_rep,
+        fused_test_add<POT>(p, wi, near, slots[(ptrdiff_t)o * FUSED_SLOTS + (k - ss)], rc2_att, rc2_rep,
                             ff, acc);
     }
     if (n_ovf && valid) {
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(fused_threads(S * G), MINB)
       for (int it = 0; it < 27; ++it) {
         const uint32_t n = min(cnt[off[it]], (uint32_t)FUSED_CAP);
         for (uint32_t k = sub; k < n; k += L)
-          mates += bead_cell(slots[(ptrdiff_t)off[it] * FUSED_CAP + k - ss], s, esc) == bead_cell(p, s, esc);
+          mates += bead_cell(slots[(ptrdiff_t)off[it] * FUSED_SLOTS + k - ss], s, esc) == bead_cell(p, s, esc);
       }
 #pragma unroll
       for (int o = L / 2; o > 0; o >>= 1)
