@@ -1096,7 +1096,9 @@ struct Engine {
 
   // Device ms per Heun step with the current grids (graphs of `reps` steps).
   double time_steps(int reps) {
-    run_steps(reps, MODE_DST, 0);  // builds the graph
+    // builds the graphs: the bucket path's count arrays are in another phase
+    // after each run, with a graph of its own, and back in the first after three
+    for (int k = 0; k < (fused ? 3 : 1); ++k) run_steps(reps, MODE_DST, 0);
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
