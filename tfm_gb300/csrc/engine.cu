@@ -1126,10 +1126,36 @@ struct Engine {
     if (par.pair_kernel != 2 && par.pair_kernel != 4)
       throw Error(ST_ARG, "autotune needs a half-shell pair kernel");
     const bool had_buckets = fused;
-    fused = false;
+    const int kernel0 = par.pair_kernel, lanes0 = par.pair_lanes, tile0 = tile;
+    std::vector<float> csl0;
+    for (const SysDesc &d : hsys) csl0.push_back(d.csl);
     download_positions();
     PinnedFloats saved_xyz = hxyz;
     uint64_t saved_step = step;
+    try {
+      fused = false;
+      std::string rep = tune(reps, csl0, had_buckets);
+      hxyz = saved_xyz;
+      upload_positions();
+      step = saved_step;
+      return rep;
+    } catch (...) {  // the batch steps as it did before
+      par.pair_kernel = kernel0;
+      par.pair_lanes = lanes0;
+      fused = had_buckets;
+      hxyz = saved_xyz;
+      step = saved_step;
+      try {
+        regrid(csl0, tile0);
+        upload_positions();
+      } catch (...) {  // the device itself fails: the first error says so
+      }
+      throw;
+    }
+  }
+
+  // The search; leaves the positions and the step wherever its runs end.
+  std::string tune(int reps, const std::vector<float> &csl0, bool had_buckets) {
     const int ns = (int)hsys.size();
     std::vector<int> cls(ns);
     std::map<int, std::vector<int>> members;
@@ -1139,8 +1165,6 @@ struct Engine {
       cls[s] = k;
       members[k].push_back(s);
     }
-    std::vector<float> csl0(ns);
-    for (int s = 0; s < ns; ++s) csl0[s] = hsys[s].csl;
     const float factors[] = {1.0f, 0.5f, 0.55f, 0.625f, 0.75f};
     struct Choice {
       int kernel;
@@ -1218,9 +1242,6 @@ struct Engine {
       fused = ms < best;
       if (fused) best = ms;
     }
-    hxyz = saved_xyz;
-    upload_positions();
-    step = saved_step;
     rep << "], \"tile\": " << best_tile << ", \"lanes\": " << best_lanes
         << ", \"buckets\": " << (fused ? 1 : 0) << ", \"tiles_tried\": [" << tt.str() << "], \"ms_per_step\": " << best << "}";
     return rep.str();
