@@ -150,7 +150,9 @@ int ccpgpu_stream_handle(ccpgpu_sim *h, void **stream);
  * observation), measured with CUDA events around individual launches on the
  * handle's stream over reps steps: out[0] scan (3 launches), [1] scatter,
  * [2] pair, [3] update stage 1, [4] update stage 2, [5] contacts,
- * [6] observe. Leaves the simulation state advanced by reps steps. */
+ * [6] observe. A batch on the bucket path, whose Heun stage is one kernel:
+ * [0] and [1] are the observation's sort, [2] is 0, [3] and [4] are the two
+ * stages. Leaves the simulation state advanced by reps steps. */
 int ccpgpu_kernel_times(ccpgpu_sim *h, int32_t reps, double *out, size_t n);
 
 /* Autotuner (no reference counterpart): for each half-shell pair kernel (2:
@@ -159,10 +161,12 @@ int ccpgpu_kernel_times(ccpgpu_sim *h, int32_t reps, double *out, size_t n);
  * 0.75, 0.625, 0.55 and 0.5 times the largest cutoff (the last four with the
  * 5x5x5 stencil), keeps the fastest per class, keeps the faster kernel, then
  * picks the per-bead tile size (64, 128, 256) and the lanes per bead (1, 2,
- * 4, 8; tile x lanes <= 512). Requires pair_kernel 2 or 4. Each
- * candidate runs reps steps; positions, time and the noise counter are
- * restored afterwards. report receives a NUL-terminated JSON summary (size in
- * *len; CCPGPU_ERR_IO when cap is too small, after tuning). */
+ * 4, 8; tile x lanes <= 512); a batch on the bucket path keeps it where it is
+ * faster than the best of these ("buckets" in the report). Requires pair_kernel
+ * 2 or 4. Each candidate runs reps steps; positions, time and the noise counter
+ * are restored afterwards, and after an error everything else too. report
+ * receives a NUL-terminated JSON summary (size in *len; CCPGPU_ERR_IO when cap
+ * is too small, after tuning). */
 int ccpgpu_autotune(ccpgpu_sim *h, int32_t reps, char *report, size_t cap, size_t *len);
 
 /* Number of engine kernels launched since creation (graph nodes included). */

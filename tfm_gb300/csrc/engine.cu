@@ -1248,16 +1248,50 @@ struct Engine {
   }
 
   // Per-kernel device times of `reps` observed steps, each kernel bracketed by
-  // its own pair of events on the engine stream.
+  // its own pair of events on the engine stream. A batch on the bucket path sorts
+  // for the observation only and its stages are one kernel each: no pair pass,
+  // the stages in the places of the update passes.
   void kernel_times(int reps, double *out) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     cudaEvent_t e[11];
     for (auto &x : e) CK(cudaEventCreate(&x));
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     set_device_step();
-    if (!hist_valid) count_cells();
-    buckets_valid = false;
+    if (fused)
+      build_buckets();
+    else if (!hist_valid)
+      count_cells();
+    buckets_valid = false;  // until every step is enqueued
     for (int r = 0; r < reps; ++r) {
+      if (fused) {
+        if (!hist_valid) count_cells();
+        CK(cudaEventRecord(e[0], stream));
+        launch_scan(false);
+        CK(cudaEventRecord(e[1], stream));
+        launch_scatter(pos.p);
+        CK(cudaEventRecord(e[2], stream));
+        launch_contacts();
+        CK(cudaEventRecord(e[3], stream));
+        launch_observe();
+        CK(cudaEventRecord(e[4], stream));
+        launch_fused<1>(fphase, false);
+        CK(cudaEventRecord(e[5], stream));
+        launch_fused<2>(fphase + 1, false);
+        CK(cudaEventRecord(e[6], stream));
+        hist_valid = false;
+        fphase = (fphase + 2) % 3;
+        CK(cudaEventSynchronize(e[6]));
+        const int at[6] = {0, 1, 5, 6, 3, 4};  // scan, scatter, contacts, observe, stages
+        for (int k = 0; k < 6; ++k) {
+          float t;
+          CK(cudaEventElapsedTime(&t, e[k], e[k + 1]));
+          acc[at[k]] += t;
+        }
+        ++step;
+        ++dev_next;
+        ++frames_observed;
+        continue;
+      }
       CK(cudaEventRecord(e[0], stream));
       launch_scan(true);
       CK(cudaEventRecord(e[1], stream));
@@ -1293,6 +1327,7 @@ struct Engine {
       ++dev_next;
       ++frames_observed;
     }
+    buckets_valid = fused;
     for (auto &x : e) cudaEventDestroy(x);
     for (int k = 0; k < 7; ++k) out[k] = acc[k] / reps;
     sync_and_check();
