@@ -62,10 +62,22 @@ struct DevBuf {
 
 constexpr int TILE = 128;
 constexpr int SMALL_BATCH = 16384;  // beads: below, tiles of 64 and 8 lanes per bead
-// Batches up to this many beads step through k_fused (fused.cuh). us per step,
-// sorted path / k_fused: ccp 98304 beads 67.1 / 58.6 (more was not measured);
-// baseline 32768 beads 56.6 / 46.6, 65536 beads 73.0 / 85.0.
+// Batches up to this many beads have buckets (fused.cuh) and take their forces
+// through them: us a call with its copies, sorted path / k_fused<0>, baseline
+// 45000 beads 122 / 80, ccp 99999 beads 162 / 90.
 constexpr int FUSED_MAX_WF = 100000, FUSED_MAX_LJ = 45000;
+// They step through them where the sum over beads of 1 + slope * packing
+// fraction stays below a limit: the full stencil's pair tests grow with both,
+// the sorted path's launches with neither. us per step, sorted path (before its
+// kernels were dependents) / k_fused, fresh states (after 18000 steps the second
+// is 5-20 % less), baseline: packing fraction 0.02, 42500 beads 60 / 52; 0.1,
+// 32785 59 / 51 and 38571 60 / 63; 0.2, 25500 60 / 58 and 30000 62 / 65; 0.25,
+// 22950 63 / 64; 0.4, 17653 67 / 47 and 20769 68 / 69. ccp: 0.02, 73010 66 / 57; 0.1,
+// 52777 53 / 54; 0.15, 44986 53 / 50 and 52924 55 / 60; 0.25, 34731 48 / 43 and
+// 40860 53 / 52. Batches at the limit: baseline 300 x 100 beads 58 / 50, 29 x
+// 1024 63 / 58; ccp 166 x 400 65 / 59, 14 x 4000 53 / 58.
+constexpr double FUSED_LOAD_WF = 78000, FUSED_LOAD_LJ = 44000;
+constexpr double FUSED_SLOPE_WF = 5.3, FUSED_SLOPE_LJ = 4.0;
 constexpr int64_t FUSED_MAX_CELLS = 1 << 19;  // 1 KB a cell
 constexpr int MAX_CPS = 1024;  // cells per side of one system's grid
 constexpr uint32_t MAX_BATCH_BEADS = (1u << (32u - BF_BITS)) - 1u;
@@ -178,7 +190,8 @@ struct Engine {
   size_t persist_bytes = 0;
   DevBuf<PGrid> d_pgrid;
   // bucket path of small batches (fused.cuh)
-  bool fused = false;
+  bool bucketed = false;               // the buckets are there: forces take them
+  bool fused = false;                  // and the steps
   int fused_lanes = 8;                 // lanes per bead
   int f_nc = 0, f_tiles = 0;           // bucket cells of all systems, CTAs
   int fphase = 0;                      // count array (of three) that holds pos
@@ -375,10 +388,11 @@ struct Engine {
     CK(cudaMemsetAsync(lbs_start.p, 0, sizeof(uint32_t) * (nc + 1), stream));
     reset_observables();
     setup_persist();
-    fused = !par.pair_path_given && persist_reach == 0 &&
-            nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) && buckets_cover_sort() &&
-            fused_cells(nullptr) <= FUSED_MAX_CELLS;
+    bucketed = !par.pair_path_given && persist_reach == 0 &&
+               nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) && buckets_cover_sort() &&
+               fused_cells(nullptr) <= FUSED_MAX_CELLS;
     setup_fused();
+    fused = bucketed && bucket_steps_pay();
     CK(cudaStreamSynchronize(stream));
   }
 
@@ -393,6 +407,18 @@ struct Engine {
     for (const SysDesc &d : hsys)
       if (!(d.csl <= bucket_side())) return false;
     return true;
+  }
+
+  // The rule at FUSED_LOAD_WF. Packing fractions are those of beads of diameter
+  // one in the nucleus (without a bleb).
+  bool bucket_steps_pay() const {
+    const bool wf = ff.pot == POT_WF;
+    double load = 0.0;
+    for (const SysDesc &d : hsys) {
+      const double phi = 0.125 * d.n / ((double)d.R_n * d.R_n * d.R_n);
+      load += d.n * (1.0 + (wf ? FUSED_SLOPE_WF : FUSED_SLOPE_LJ) * phi);
+    }
+    return load <= (wf ? FUSED_LOAD_WF : FUSED_LOAD_LJ);
   }
 
   // Bucket grids of all systems. Returns the number of cells.
@@ -411,10 +437,10 @@ struct Engine {
   }
 
   // Sets the bucket path up (with the other buffers: a first call does not pay
-  // for it); the batch steps through the sorted path when there is no memory
-  // left for the buckets.
+  // for it); the batch goes through the sorted path when there is no memory left
+  // for the buckets.
   void setup_fused() {
-    if (!fused) return;
+    if (!bucketed) return;
     std::vector<FusedGrid> g;
     f_nc = (int)fused_cells(&g);
     // More lanes per bead shorten a kernel until its CTAs (256 / lanes beads,
@@ -451,7 +477,7 @@ struct Engine {
       }
       fcnt.release();
       d_ftiles.release();
-      fused = false;
+      bucketed = false;
       return;
     }
     CK(cudaMemcpyAsync(d_ftiles.p, tl.data(), sizeof(Tile) * tl.size(), cudaMemcpyHostToDevice,
@@ -1125,7 +1151,7 @@ struct Engine {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     if (par.pair_kernel != 2 && par.pair_kernel != 4)
       throw Error(ST_ARG, "autotune needs a half-shell pair kernel");
-    const bool had_buckets = fused;
+    const bool fused0 = fused;
     const int kernel0 = par.pair_kernel, lanes0 = par.pair_lanes, tile0 = tile;
     std::vector<float> csl0;
     for (const SysDesc &d : hsys) csl0.push_back(d.csl);
@@ -1134,7 +1160,7 @@ struct Engine {
     uint64_t saved_step = step;
     try {
       fused = false;
-      std::string rep = tune(reps, csl0, had_buckets);
+      std::string rep = tune(reps, csl0);
       hxyz = saved_xyz;
       upload_positions();
       step = saved_step;
@@ -1142,7 +1168,7 @@ struct Engine {
     } catch (...) {  // the batch steps as it did before
       par.pair_kernel = kernel0;
       par.pair_lanes = lanes0;
-      fused = had_buckets;
+      fused = fused0;
       hxyz = saved_xyz;
       step = saved_step;
       try {
@@ -1155,7 +1181,7 @@ struct Engine {
   }
 
   // The search; leaves the positions and the step wherever its runs end.
-  std::string tune(int reps, const std::vector<float> &csl0, bool had_buckets) {
+  std::string tune(int reps, const std::vector<float> &csl0) {
     const int ns = (int)hsys.size();
     std::vector<int> cls(ns);
     std::map<int, std::vector<int>> members;
@@ -1235,8 +1261,10 @@ struct Engine {
     }
     par.pair_lanes = best_lanes;
     regrid(csl, best_tile);
-    // the bucket path stays where it is faster than the best of these
-    if (had_buckets && buckets_cover_sort()) {
+    // the buckets go where they no longer cover the sort's cells; the steps take
+    // them where they are faster than the best of these
+    bucketed = bucketed && buckets_cover_sort();
+    if (bucketed) {
       fused = true;
       const double ms = time_steps(reps);
       fused = ms < best;
@@ -1582,7 +1610,7 @@ struct Engine {
   // is written only when the state is not refused.
   void forces(float *f) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
-    if (fused) {
+    if (bucketed) {
       build_buckets();
       launch_fused<0>(fphase, false);
     } else {
