@@ -779,6 +779,20 @@ struct Engine {
     kcount += 1;
   }
   bool chain_open = false;  // capturing a chain
+  // A dependent's CTAs go to the SMs that the kernel before leaves first. Where
+  // the whole grid fits on a part of the GPU it piles up there and the other SMs
+  // idle: the update pass of a few waves (tiles of 64 and 128), and with tiles of
+  // 128 the pair pass too, wait for the end of the kernel before instead. Smaller
+  // batches are bound by latency, larger ones refill the SMs. us per step: all
+  // dependent / none / by this rule: ccp 500 x 190 beads 76.4 / 67.9 / 67.4, 99999
+  // beads 74.1 / 70.4 / 68.3; baseline 20 x 5000 96.7 / 92.0 / 88.6, 60 x 5000
+  // (tiles of 128) 171.8 / 167.2 / 164.2, 131072 93.2 / 97.2 / 94.4; outside it,
+  // all dependent / none: ccp 36000 43.6 / 46.8, 2500 x 100 131.0 / 136.2, baseline
+  // 8000 48.1 / 51.2, 1500 x 200 176.9 / 194.1, 250 x 6000 541.7 / 551.9.
+  bool piles_up() const {
+    const size_t threads = htiles.size() * (size_t)tile;
+    return threads >= 40960 && threads < 320000;
+  }
 
   void launch_scan(bool bump) {
     launch(k_scan_reduce, nblk, SCAN_THREADS, counts.p, bsum.p);
@@ -860,6 +874,7 @@ struct Engine {
 
   template <int MODE>
   void launch_pair() {
+    if (piles_up() && tile >= 128) chained = false;
     const unsigned nt = (unsigned)htiles.size();
     if (par.pair_kernel == 4) {
       switch (typed_reaches<MODE>()) {
@@ -923,6 +938,7 @@ struct Engine {
 
   template <int STAGE, int MODE>
   void launch_update() {
+    if (piles_up()) chained = false;
     launch(k_update<STAGE, MODE>, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, ff, pos.p,
            er.p, fbuf.p, rnb.p, fs.p, rank.p, counts.p, lbs_sorted.p, lbs_start.p, d_step.p,
            d_err.p);
