@@ -43,7 +43,7 @@ def test_rule(engine_lib, preset, sizes, phi, kernels):
     b.close()
 
 
-# on both sides of the line, and with four lanes a bead (ccp above 49152)
+# on both sides of the line, and the largest batches that step through buckets
 @pytest.mark.parametrize("preset,n,phi", [("baseline", 24000, 0.2), ("baseline", 25000, 0.2),
                                           ("ccp", 67000, 0.03), ("ccp", 47000, 0.13)])
 def test_steps_and_forces_as_the_sorted_path(engine_lib, preset, n, phi):

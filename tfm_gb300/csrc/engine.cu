@@ -445,17 +445,17 @@ struct Engine {
     f_nc = (int)fused_cells(&g);
     // More lanes per bead shorten a kernel until its CTAs (256 / lanes beads,
     // three or four on an SM) no longer fit the GPU at once. us per step with
-    // 32 / 16 / 8 lanes, baseline: 2048 beads 12.2 / 16.2 / 26.2, 4096 beads
-    // 19.5 / 15.9 / 24.5, 8192 beads 28.7 / 25.6 / 25.1, 32768 beads - / 62.8 /
-    // 46.6; ccp: 2048 beads 9.0 / 9.5 / 13.3, 4096 beads 14.3 / 10.0 / 13.0,
-    // 8192 beads 20.4 / 15.7 / 13.9. Four lanes pay with ccp's small cells
-    // only: 32768 beads 26.3 (8) / 29.0 (4), 65536 beads 47.8 / 44.3.
+    // 32 / 16 / 8 lanes, ccp (packing fraction 0.08): 2048 beads 10.8 / 12.1 /
+    // 16.5, 3648 10.9 / 11.8 / 15.1, 4096 15.0 / 12.3 / 15.9, 7296 18.7 / 12.7 / 16.3,
+    // 8192 23.3 / 18.4 / 17.9, 32768 69.7 / 45.8 / 33.5; baseline (0.2): 2048 beads
+    // 13.5 / 18.4 / 28.1, 3648 14.0 / 18.9 / 29.6, 4096 22.4 / 20.8 / 33.3, 8192 31.0 /
+    // 29.0 / 31.3, 16384 53.6 / 45.4 / 36.9. Four lanes: ccp 32768 beads 38.7,
+    // 65536 61.3 (58.5 with eight).
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t fit = (int64_t)3 * sms * FUSED_PAIR_THREADS;
     fused_lanes = (int64_t)nb * 32 <= fit ? 32 : ((int64_t)nb * 16 <= fit ? 16 : 8);
-    if (ff.pot == POT_WF && nb > 49152) fused_lanes = 4;
     const int per = FUSED_PAIR_THREADS / fused_lanes;
     std::vector<Tile> tl;
     for (int s = 0; s < (int)hsys.size(); ++s)
@@ -541,10 +541,8 @@ struct Engine {
         CCPGPU_FUSED(POT_WF, 4, 8, 3);
       else if (fused_lanes == 16)
         CCPGPU_FUSED(POT_WF, 4, 4, 3);
-      else if (fused_lanes == 8)
-        CCPGPU_FUSED(POT_WF, 4, 2, 4);
       else
-        CCPGPU_FUSED(POT_WF, 4, 1, 3);
+        CCPGPU_FUSED(POT_WF, 4, 2, 4);
     } else {
       if (fused_lanes == 32)
         CCPGPU_FUSED(POT_LJ, 8, 4, 3);
