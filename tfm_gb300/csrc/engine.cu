@@ -1466,8 +1466,8 @@ struct Engine {
   // The device's error flags; clear also forgets the histogram and the buckets,
   // so that the next call counts again and flags what is still wrong.
   void read_flags(int *e, bool clear) {
+    CK(cudaMemcpyAsync(e, d_err.p, sizeof(int) * ERR_COUNT, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    CK(cudaMemcpy(e, d_err.p, sizeof(int) * ERR_COUNT, cudaMemcpyDeviceToHost));
     if (!clear) return;
     CK(cudaMemsetAsync(d_err.p, 0, sizeof(int) * ERR_COUNT, stream));
     if (e[ERR_ESCAPE] || e[ERR_SLOT]) hist_valid = buckets_valid = false;
