@@ -12,11 +12,10 @@
 // stencil, which is what ends the range of this path.
 //
 // Measured on a GB300, us per Heun step, sorted path / this one (single
-// systems at ccp's chromatin volume fraction 0.125, baseline at packing
-// fraction 0.2):
-//   beads          1024         2048         8192         32768        98304
-//   ccp        38.4 /  8.6  39.8 /  9.0  41.7 / 13.6  47.9 / 26.3  68.3 / 58.6
-//   baseline   44.6 / 11.9  45.9 / 12.2  49.3 / 24.9  56.3 / 46.9  81.4 / 118
+// systems at packing fraction 0.08, ccp, and 0.2, baseline):
+//   beads          1024         2048         8192         24000        40000
+//   ccp        35.3 /  8.9  38.7 / 10.8  41.6 / 17.9  48.2 / 28.6  52.8 / 42.1
+//   baseline   43.0 / 12.9  42.0 / 13.5  45.9 / 31.4  58.4 / 59.9  62.1 / 75.4
 //
 // Buckets. Every system has a grid of cells of side the largest pair cutoff.
 // A cell holds up to FUSED_CAP (x, y, z, index << 3 | flags) slots; beads
@@ -28,7 +27,7 @@
 // CTA: 8 warps of pair lanes (L = S G lanes a bead, 256 / L beads), which also
 // take the lamina sites, and two threads a bead that meanwhile compute its
 // bonded and wall forces and its noise (one thread a bead for all of these,
-// sites included, took 12.9 instead of 9.5 us a step at 1024 ccp beads: its
+// sites included, took 12.9 instead of 9.5 us a step at 1024 ccp beads then: its
 // serial chain was longer than the pair loop).
 #pragma once
 
