@@ -69,15 +69,26 @@ constexpr int FUSED_MAX_WF = 100000, FUSED_MAX_LJ = 45000;
 // They step through them where the sum over beads of 1 + slope * packing
 // fraction stays below a limit: the full stencil's pair tests grow with both,
 // the sorted path's launches with neither. us per step, sorted path (before its
-// kernels were dependents) / k_fused, fresh states (after 18000 steps the second
-// is 5-20 % less), baseline: packing fraction 0.02, 42500 beads 60 / 52; 0.1,
-// 32785 59 / 51 and 38571 60 / 63; 0.2, 25500 60 / 58 and 30000 62 / 65; 0.25,
-// 22950 63 / 64; 0.4, 17653 67 / 47 and 20769 68 / 69. ccp: 0.02, 73010 66 / 57; 0.1,
-// 52777 53 / 54; 0.15, 44986 53 / 50 and 52924 55 / 60; 0.25, 34731 48 / 43 and
-// 40860 53 / 52. Batches at the limit: baseline 300 x 100 beads 58 / 50, 29 x
-// 1024 63 / 58; ccp 166 x 400 65 / 59, 14 x 4000 53 / 58.
+// kernels were dependents) / k_fused, states fresh from the relaxation (after
+// 18000 steps the second is 5-20 % less), baseline: packing fraction 0.02, 42500
+// beads 60 / 52; 0.1, 32785 59 / 51 and 38571 60 / 63; 0.2, 25500 60 / 58 and
+// 30000 62 / 65; 0.25, 22950 63 / 64; 0.4, 17653 67 / 47 and 20769 68 / 69. ccp:
+// 0.02, 73010 66 / 57; 0.1, 52777 53 / 54; 0.15, 44986 53 / 50 and 52924 55 / 60;
+// 0.25, 34731 48 / 43 and 40860 53 / 52.
 constexpr double FUSED_LOAD_WF = 78000, FUSED_LOAD_LJ = 44000;
 constexpr double FUSED_SLOPE_WF = 5.3, FUSED_SLOPE_LJ = 4.0;
+// Beyond that limit by the state that the steps start from: while at most this
+// share of the beads is in cells with more than fused_read of them (and a
+// baseline batch is at most two waves of CTAs). A walk folds into a coil whose
+// density varies from cell to cell, and keeps it for long; evenly spread beads
+// do not leave the fast loop. us per step, sorted path / k_fused, share: ccp,
+// evenly spread at packing fraction 0.12, 57450 beads 50 / 38, 0.01 (53 / 40, 0.11
+// after 6000 steps), 99000 63 / 61, 0.01; walks at 0.03, 74000 beads 65 / 53, 0.23;
+// at 0.08, 70000 60 / 64, 0.47 (59 / 58, 0.33); at 0.13, 56000 53 / 59, 0.64;
+// baseline, evenly spread at 0.2, 36735 beads 55 / 45, 0.05 (58 / 50, 0.23), 44900
+// 56 / 59; walks at 0.1, 33000 beads 58 / 54, 0.30 (57 / 47, 0.16); at 0.15, 34000 61 /
+// 67, 0.46 (59 / 60, 0.32).
+constexpr double FUSED_CROWD = 0.25;
 constexpr int64_t FUSED_MAX_CELLS = 1 << 19;  // 1 KB a cell
 constexpr int MAX_CPS = 1024;  // cells per side of one system's grid
 constexpr uint32_t MAX_BATCH_BEADS = (1u << (32u - BF_BITS)) - 1u;
@@ -192,6 +203,8 @@ struct Engine {
   // bucket path of small batches (fused.cuh)
   bool bucketed = false;               // the buckets are there: forces take them
   bool fused = false;                  // and the steps
+  bool by_state = false;               // ... as the positions' spread decides
+  bool state_known = false;            // ... which has been looked at
   int fused_lanes = 8;                 // lanes per bead
   int f_nc = 0, f_tiles = 0;           // bucket cells of all systems, CTAs
   int fphase = 0;                      // count array (of three) that holds pos
@@ -201,6 +214,7 @@ struct Engine {
   DevBuf<Tile> d_ftiles;
   DevBuf<float4> fslots[2], fovf[2];
   DevBuf<uint32_t> fcnt;
+  DevBuf<unsigned int> d_crowd;
 
   ~Engine() {
     for (auto &g : graphs) cudaGraphExecDestroy(g.second);
@@ -391,8 +405,9 @@ struct Engine {
     bucketed = !par.pair_path_given && persist_reach == 0 &&
                nb <= (ff.pot == POT_WF ? FUSED_MAX_WF : FUSED_MAX_LJ) && buckets_cover_sort() &&
                fused_cells(nullptr) <= FUSED_MAX_CELLS;
-    setup_fused();
     fused = bucketed && bucket_steps_pay();
+    by_state = bucketed && !fused && (ff.pot == POT_WF || nb <= 2 * fused_wave());
+    setup_fused();
     CK(cudaStreamSynchronize(stream));
   }
 
@@ -419,6 +434,31 @@ struct Engine {
       load += d.n * (1.0 + (wf ? FUSED_SLOPE_WF : FUSED_SLOPE_LJ) * phi);
     }
     return load <= (wf ? FUSED_LOAD_WF : FUSED_LOAD_LJ);
+  }
+
+  // Beads of a wave of k_fused's CTAs with eight lanes a bead, four on an SM.
+  static int fused_wave() {
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms * 4 * FUSED_PAIR_THREADS / 8;
+  }
+
+  // The rule at FUSED_CROWD, for positions that no earlier call has looked at:
+  // a few microseconds on the device and a wait for the count.
+  void choose_path() {
+    if (!by_state || state_known) return;
+    build_buckets();
+    unsigned int crowd = 0;
+    CK(cudaMemsetAsync(d_crowd.p, 0, sizeof(crowd), stream));
+    k_fused_crowd<<<(unsigned)std::min(152, (f_nc + 255) / 256), 256, 0, stream>>>(
+        fcnt.p + ((size_t)f_nc + 1) * (fphase % 3), f_nc, (uint32_t)fused_read(ff.pot), d_crowd.p);
+    CK(cudaGetLastError());
+    kcount += 1;
+    CK(cudaMemcpyAsync(&crowd, d_crowd.p, sizeof(crowd), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    fused = crowd <= FUSED_CROWD * nb;
+    state_known = true;
   }
 
   // Bucket grids of all systems. Returns the number of cells.
@@ -449,13 +489,15 @@ struct Engine {
     // 16.5, 3648 10.9 / 11.8 / 15.1, 4096 15.0 / 12.3 / 15.9, 7296 18.7 / 12.7 / 16.3,
     // 8192 23.3 / 18.4 / 17.9, 32768 69.7 / 45.8 / 33.5; baseline (0.2): 2048 beads
     // 13.5 / 18.4 / 28.1, 3648 14.0 / 18.9 / 29.6, 4096 22.4 / 20.8 / 33.3, 8192 31.0 /
-    // 29.0 / 31.3, 16384 53.6 / 45.4 / 36.9. Four lanes: ccp 32768 beads 38.7,
-    // 65536 61.3 (58.5 with eight).
+    // 29.0 / 31.3, 16384 53.6 / 45.4 / 36.9. Four lanes pay for the evenly spread
+    // states alone that FUSED_CROWD admits: eight / four, ccp, 57450 beads 39.5 /
+    // 35.1, 75081 51.0 / 47.7, but walks, 56000 beads 53.6 / 59.0, 65536 58.5 / 61.3.
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t fit = (int64_t)3 * sms * FUSED_PAIR_THREADS;
     fused_lanes = (int64_t)nb * 32 <= fit ? 32 : ((int64_t)nb * 16 <= fit ? 16 : 8);
+    if (by_state && ff.pot == POT_WF && nb > 49152) fused_lanes = 4;
     const int per = FUSED_PAIR_THREADS / fused_lanes;
     std::vector<Tile> tl;
     for (int s = 0; s < (int)hsys.size(); ++s)
@@ -469,6 +511,7 @@ struct Engine {
       fcnt.alloc((size_t)3 * (f_nc + 1));
       d_ftiles.alloc(tl.size());
       d_fgrid.alloc(g.size());
+      d_crowd.alloc(1);
     } catch (const Error &) {
       cudaGetLastError();
       for (int k = 0; k < 2; ++k) {
@@ -477,7 +520,7 @@ struct Engine {
       }
       fcnt.release();
       d_ftiles.release();
-      bucketed = false;
+      bucketed = fused = by_state = false;
       return;
     }
     CK(cudaMemcpyAsync(d_ftiles.p, tl.data(), sizeof(Tile) * tl.size(), cudaMemcpyHostToDevice,
@@ -535,21 +578,23 @@ struct Engine {
     c.attrs = &at;
     c.numAttrs = dependent ? 1 : 0;
 #define CCPGPU_FUSED(POT, S, G, MINB) CK(cudaLaunchKernelEx(&c, k_fused<STAGE, POT, S, G, MINB>, a, ff))
-    // S: cells hold 2-3 beads in ccp's field (side 2), 6 in the baseline (2.5)
+    constexpr int SW = fused_read(POT_WF), SL = fused_read(POT_LJ);
     if (ff.pot == POT_WF) {
       if (fused_lanes == 32)
-        CCPGPU_FUSED(POT_WF, 4, 8, 3);
+        CCPGPU_FUSED(POT_WF, SW, 8, 3);
       else if (fused_lanes == 16)
-        CCPGPU_FUSED(POT_WF, 4, 4, 3);
+        CCPGPU_FUSED(POT_WF, SW, 4, 3);
+      else if (fused_lanes == 8)
+        CCPGPU_FUSED(POT_WF, SW, 2, 4);
       else
-        CCPGPU_FUSED(POT_WF, 4, 2, 4);
+        CCPGPU_FUSED(POT_WF, SW, 1, 3);
     } else {
       if (fused_lanes == 32)
-        CCPGPU_FUSED(POT_LJ, 8, 4, 3);
+        CCPGPU_FUSED(POT_LJ, SL, 4, 3);
       else if (fused_lanes == 16)
-        CCPGPU_FUSED(POT_LJ, 8, 2, 3);
+        CCPGPU_FUSED(POT_LJ, SL, 2, 3);
       else
-        CCPGPU_FUSED(POT_LJ, 8, 1, 4);
+        CCPGPU_FUSED(POT_LJ, SL, 1, 4);
     }
 #undef CCPGPU_FUSED
     kcount += 1;
@@ -685,7 +730,7 @@ struct Engine {
   }
 
   void recount() {
-    buckets_valid = false;  // the positions have changed
+    buckets_valid = state_known = false;  // the positions have changed
     count_cells();
   }
 
@@ -1165,7 +1210,7 @@ struct Engine {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
     if (par.pair_kernel != 2 && par.pair_kernel != 4)
       throw Error(ST_ARG, "autotune needs a half-shell pair kernel");
-    const bool fused0 = fused;
+    const bool fused0 = fused, by_state0 = by_state;
     const int kernel0 = par.pair_kernel, lanes0 = par.pair_lanes, tile0 = tile;
     std::vector<float> csl0;
     for (const SysDesc &d : hsys) csl0.push_back(d.csl);
@@ -1173,7 +1218,7 @@ struct Engine {
     PinnedFloats saved_xyz = hxyz;
     uint64_t saved_step = step;
     try {
-      fused = false;
+      fused = by_state = false;  // the search decides
       std::string rep = tune(reps, csl0);
       hxyz = saved_xyz;
       upload_positions();
@@ -1183,6 +1228,7 @@ struct Engine {
       par.pair_kernel = kernel0;
       par.pair_lanes = lanes0;
       fused = fused0;
+      by_state = by_state0;
       hxyz = saved_xyz;
       step = saved_step;
       try {
@@ -1295,6 +1341,7 @@ struct Engine {
   // the stages in the places of the update passes.
   void kernel_times(int reps, double *out) {
     if (!positions_valid) throw Error(ST_STATE, "positions not initialised");
+    choose_path();
     cudaEvent_t e[11];
     for (auto &x : e) CK(cudaEventCreate(&x));
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -1394,6 +1441,10 @@ struct Engine {
     }
     set_device_step();
     if (n == 0) return;
+    if (mode == MODE_DST)
+      choose_path();
+    else
+      state_known = false;
     const bool buckets = fused && mode == MODE_DST;
     if (buckets) {
       build_buckets();

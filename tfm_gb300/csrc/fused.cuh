@@ -109,6 +109,22 @@ __global__ void k_fused_build(const Tile *__restrict__ tiles, const SysDesc *__r
   fused_insert(pos[i], i, s, grid[t.sys], cnt, slots, ovf, n_cells, err);
 }
 
+// Slots of a cell that the lanes of a bead read together; the beads beyond them
+// take a loop of their own. Cells hold 2-3 beads in ccp's field (side 2), 6 in
+// the baseline (2.5).
+__host__ __device__ constexpr int fused_read(int pot) { return pot == POT_WF ? 4 : 8; }
+
+// Number of beads in cells that hold more than `most`, added to *sum.
+__global__ void __launch_bounds__(256)
+    k_fused_crowd(const uint32_t *__restrict__ cnt, int n_cells, uint32_t most,
+                  unsigned int *__restrict__ sum) {
+  unsigned int s = 0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cells; c += gridDim.x * blockDim.x)
+    s += cnt[c] > most ? cnt[c] : 0u;
+  s = __reduce_add_sync(0xffffffffu, s);
+  if ((threadIdx.x & 31u) == 0u && s) atomicAdd(sum, s);
+}
+
 // Whether the pair of the bead at p (word wi, `near` = (index - 1) << 3) and
 // the candidate q is within its class's cutoff and not |i - j| <= 1.
 __device__ __forceinline__ bool fused_hit(float4 p, uint32_t wi, uint32_t near, float4 q,
