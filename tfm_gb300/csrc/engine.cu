@@ -824,17 +824,18 @@ struct Engine {
   bool chain_open = false;  // capturing a chain
   // A dependent's CTAs go to the SMs that the kernel before leaves first. Where
   // the whole grid fits on a part of the GPU it piles up there and the other SMs
-  // idle: the update pass of a few waves (tiles of 64 and 128), and with tiles of
-  // 128 the pair pass too, wait for the end of the kernel before instead. Smaller
-  // batches are bound by latency, larger ones refill the SMs. us per step: all
-  // dependent / none / by this rule: ccp 500 x 190 beads 76.4 / 67.9 / 67.4, 99999
-  // beads 74.1 / 70.4 / 68.3; baseline 20 x 5000 96.7 / 92.0 / 88.6, 60 x 5000
-  // (tiles of 128) 171.8 / 167.2 / 164.2, 131072 93.2 / 97.2 / 94.4; outside it,
-  // all dependent / none: ccp 36000 43.6 / 46.8, 2500 x 100 131.0 / 136.2, baseline
-  // 8000 48.1 / 51.2, 1500 x 200 176.9 / 194.1, 250 x 6000 541.7 / 551.9.
+  // idle: in batches of a few waves the update pass waits for the end of the
+  // kernel before instead, and with it the scatter (tiles of 64) or the pair pass
+  // (tiles of 128). Smaller batches are bound by latency, larger ones refill the
+  // SMs. us per step, all dependent / none / by this rule: ccp 500 x 190 beads 76.4
+  // / 67.9 / 66; at packing fraction 0.02 73010 beads 75.0 / 65.1 / 62.5, 99000 80.1 /
+  // 76.7 / 74.4; baseline 200 x 200 beads 76.7 / 72.9 / 69.1, 90000 at 0.1 82.4 / 82.4 /
+  // 79.6, tiles of 128: 180 x 100 57.3 / - / 54.7, 60 x 5000 178 / 170 / 168; outside it, all dependent / none:
+  // ccp 24000 42.6 / 45.6, baseline 12000 48.3 / 51.4, 1500 x 200 178 / 196, 600 x
+  // 1024 271 / 273.
   bool piles_up() const {
     const size_t threads = htiles.size() * (size_t)tile;
-    return threads >= 40960 && threads < 320000;
+    return threads >= (tile < 128 ? 28672 : 20480) && threads < 320000;
   }
 
   void launch_scan(bool bump) {
@@ -844,6 +845,7 @@ struct Engine {
   }
 
   void launch_scatter(const float4 *src) {
+    if (piles_up() && tile < 128) chained = false;
     launch(k_scatter, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, src, rank.p, start.p,
            sorted.p, par.pair_kernel >= 2 ? fs.p : nullptr, counts.p, d_err.p);
   }
