@@ -328,8 +328,17 @@ struct Engine {
     // 1024 68.4 / 64.1, 64 x 2000 104.8 / 99.0, 30 x 7000 132.6 / 128.6, but
     // 131072 in one system 84.0 / 89.3 (its A beads come first and fill the
     // ragged end's place), 512 replicas 898 / 915; ccp 40 x 4000 85.5 / 83.0,
-    // 128 x 1024 77.6 / 78.4.
-    tile = (nb < SMALL_BATCH || (nb < 262144 && (ns > 1 || nb < 100000))) ? 64 : TILE;
+    // 128 x 1024 77.6 / 78.4. Systems of at most 256 beads gain where the smaller
+    // tiles have fewer idle threads (225 x 400 103 / 84.9, 600 x 150 93.4 / 83.6) and
+    // lose where they have as many (900 x 100 82.7 / 97.1, 703 x 128 81.2 / 86.7, 450 x
+    // 200 98.3 / 103).
+    int64_t pad64 = 0, pad128 = 0;
+    for (const SysDesc &d : hsys) {
+      pad64 += (d.n + 63) / 64 * 64;
+      pad128 += (d.n + 127) / 128 * 128;
+    }
+    const bool wide = nb <= (int64_t)256 * ns && 20 * pad64 > 19 * pad128;
+    tile = (nb < SMALL_BATCH || (nb < 262144 && (ns > 1 || nb < 100000) && !wide)) ? 64 : TILE;
     build_tiles();
     nblk = (nc + 1 + SCAN_CHUNK - 1) / SCAN_CHUNK;
 
