@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256)
 __device__ __forceinline__ bool fused_hit(float4 p, uint32_t wi, uint32_t near, float4 q,
                                           float rc2_att, float rc2_rep) {
   const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  const float d2 = dx * dx + dy * dy + dz * dz;
+  const float d2 = pair_d2(dx, dy, dz);
   const uint32_t wj = wbits(q);
   return d2 <= ((wi & wj & BF_HET) ? rc2_att : rc2_rep) && wj - near >= (3u << BF_BITS);
 }
@@ -160,7 +160,7 @@ struct ForceSum {
 template <int POT, bool HH>
 __device__ __forceinline__ void fused_add(float4 p, float4 q, const ForceField &ff, ForceSum &acc) {
   const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  const float d2 = dx * dx + dy * dy + dz * dz;
+  const float d2 = pair_d2(dx, dy, dz);
   const float cf = POT == POT_WF ? wf_coef(ff.e_att, d2)
                                  : lj_coef<!HH>(HH ? ff.e_att : ff.e_rep, dx, dy, dz, d2);
   acc.add(cf * dx, cf * dy, cf * dz);

@@ -127,6 +127,13 @@ __device__ __forceinline__ float r_over_d_minus1(float R, float a, float b, floa
   return -sq3_minus(a, b, c, rh, rl) / ((R + d) * d);
 }
 
+// Squared length of a pair vector, formed in one order by every pair kernel: a
+// truncated force jumps at its cutoff (the Lennard-Jones one by 0.02 kT/sigma),
+// and a pair there is in or out alike on every path.
+__device__ __forceinline__ float pair_d2(float dx, float dy, float dz) {
+  return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+}
+
 // Wang-Frenkel (rc = 2) coefficient e (18 d^4 - 96 d^2 + 96) / d^8 in the
 // factored form 6 e (d^2 - 4)(3 d^2 - 4) / d^8 (roots at the cutoffs 2 and 2/sqrt(3)).
 __device__ __forceinline__ float wf_coef(float e, float d2) {
@@ -528,7 +535,7 @@ __device__ __forceinline__ void pair_accum(float4 p, uint32_t wi, float4 q, cons
   int gi = (int)(wi >> BF_BITS), gj = (int)(wj >> BF_BITS);
   bool excl = (unsigned)(gi - gj + 1) <= 2u;
   float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  float d2 = dx * dx + dy * dy + dz * dz;
+  float d2 = pair_d2(dx, dy, dz);
   float cf;
   if (MODE == MODE_ICG) {
     float d = sqrtf(d2);
@@ -583,7 +590,7 @@ __global__ void __launch_bounds__(256)
         uint32_t wj = wbits(q);
         int gi = (int)(wi >> BF_BITS), gj = (int)(wj >> BF_BITS);
         float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        float d2 = dx * dx + dy * dy + dz * dz;
+        float d2 = pair_d2(dx, dy, dz);
         bool hh = (wi & wj & BF_HET) != 0u;
         float rc = (MODE == MODE_ICG) ? ff.rc_icg : (hh ? ff.rc_att : ff.rc_rep);
         if (d2 > rc * rc || (unsigned)(gi - gj + 1) <= 2u) continue;
@@ -612,7 +619,7 @@ __device__ __forceinline__ void half_pair(float4 p, uint32_t wi, const float4 *_
   uint32_t wj = wbits(q);
   int gi = (int)(wi >> BF_BITS), gj = (int)(wj >> BF_BITS);
   float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  float d2 = dx * dx + dy * dy + dz * dz;
+  float d2 = pair_d2(dx, dy, dz);
   bool hh = (wi & wj & BF_HET) != 0u;
   float rc = (MODE == MODE_ICG) ? ff.rc_icg : (hh ? ff.rc_att : ff.rc_rep);
   if (d2 > rc * rc || (unsigned)(gi - gj + 1) <= 2u) return;
@@ -632,7 +639,7 @@ __device__ __forceinline__ void half_pair_q(float4 p, uint32_t wi, float4 q, uin
                                             const ForceField &ff, float rc2_max, float3 &acc,
                                             float4 *__restrict__ fs) {
   float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  float d2 = dx * dx + dy * dy + dz * dz;
+  float d2 = pair_d2(dx, dy, dz);
   if (d2 > rc2_max) return;
   uint32_t wj = wbits(q);
   bool hh = (wi & wj & BF_HET) != 0u;
@@ -724,7 +731,7 @@ __device__ __forceinline__ void typed_pair(float4 p, uint32_t wi, float4 q, uint
                                            const ForceField &ff, float rc2, float3 &acc,
                                            float4 *__restrict__ fs) {
   float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-  float d2 = dx * dx + dy * dy + dz * dz;
+  float d2 = pair_d2(dx, dy, dz);
   if (d2 > rc2) return;
   int gi = (int)(wi >> BF_BITS), gj = (int)(wbits(q) >> BF_BITS);
   if ((unsigned)(gi - gj + 1) <= 2u) return;

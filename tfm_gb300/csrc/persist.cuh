@@ -132,7 +132,7 @@ __device__ __forceinline__ void persist_pairs(const PersistSmem &m, int n, const
       for (int j = b; j < e; ++j) {
         const float4 q = m.sorted[j];
         const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        const float d2 = dx * dx + dy * dy + dz * dz;
+        const float d2 = pair_d2(dx, dy, dz);
         if (d2 > rc2_max) continue;
         const uint32_t wj = wbits(q);
         const bool hh = (wi & wj & BF_HET) != 0u;
