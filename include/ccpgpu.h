@@ -139,6 +139,8 @@ int ccpgpu_run_steps(ccpgpu_sim *h, uint64_t n_steps, uint32_t observe_every);
 /* Enqueues n_steps Heun steps on the handle's stream and returns without
  * waiting or copying positions back (the device-resident form of
  * ccpgpu_run_steps); ccpgpu_synchronize waits and checks the error flags.
+ * The first steps from new positions of a batch beyond the density limit of the
+ * bucket path wait once for a count of the crowded cells (some 10 us).
  * No reference counterpart (ccp's loop synchronises every frame, chrsim.cu:583). */
 int ccpgpu_advance(ccpgpu_sim *h, uint64_t n_steps, uint32_t observe_every);
 int ccpgpu_synchronize(ccpgpu_sim *h);
