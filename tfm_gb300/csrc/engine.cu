@@ -834,18 +834,18 @@ struct Engine {
   // A dependent's CTAs go to the SMs that the kernel before leaves first. Where
   // the whole grid fits on a part of the GPU it piles up there and the other SMs
   // idle: in batches of a few waves the update pass waits for the end of the
-  // kernel before instead, and with it the scatter (tiles of 64) or the pair pass
-  // (tiles of 128). Smaller batches are bound by latency, larger ones refill the
-  // SMs. us per step, all dependent / none / by this rule: ccp 500 x 190 beads 76.4
-  // / 67.9 / 66; at packing fraction 0.02 73010 beads 75.0 / 65.1 / 62.5, 99000 80.1 /
-  // 76.7 / 74.4; baseline 200 x 200 beads 76.7 / 72.9 / 69.1, 90000 at 0.1 82.4 / 82.4 /
-  // 79.6, tiles of 128: 180 x 100 57.3 / - / 54.7, 60 x 5000 178 / 170 / 168; outside it, all dependent / none:
-  // ccp 24000 42.6 / 45.6, baseline 12000 48.3 / 51.4, 1500 x 200 178 / 196, 600 x
-  // 1024 271 / 273.
-  bool piles_up() const {
-    const size_t threads = htiles.size() * (size_t)tile;
-    return threads >= (tile < 128 ? 28672 : 20480) && threads < 320000;
-  }
+  // kernel before instead, and with it the scatter or, in the largest of them, the
+  // pair pass. Smaller batches are bound by latency, larger ones refill the SMs.
+  // us per step, all dependent / none / by this rule: ccp 500 x 190 beads 76.4 / 67.9
+  // / 66; at packing fraction 0.02 73010 beads 75.0 / 65.1 / 62.5, 99000 80.1 / 76.7 /
+  // 74.4; baseline 200 x 200 beads 76.7 / 72.9 / 69.1, 90000 at 0.1 82.4 / 82.4 / 79.6,
+  // 131072 (evenly spread) 82.0 / 88.3 / 82.0, 60 x 5000 178 / 170 / 168; outside it, all
+  // dependent / none: ccp 24000 42.6 / 45.6, baseline 12000 48.3 / 51.4, 1500 x 200 178 /
+  // 196, 600 x 1024 271 / 273. Scatter / pair pass waiting: 131072 82.0 / 85.8, 110000
+  // 89.6 / 88.6, 220000 120 / 120, 270 x 1024 169 / 162.
+  size_t padded() const { return htiles.size() * (size_t)tile; }
+  bool piles_up() const { return padded() >= (tile < 128 ? 28672 : 20480) && padded() < 320000; }
+  bool pair_piles_up() const { return piles_up() && padded() >= 262144; }
 
   void launch_scan(bool bump) {
     launch(k_scan_reduce, nblk, SCAN_THREADS, counts.p, bsum.p);
@@ -854,7 +854,7 @@ struct Engine {
   }
 
   void launch_scatter(const float4 *src) {
-    if (piles_up() && tile < 128) chained = false;
+    if (piles_up() && !pair_piles_up()) chained = false;
     launch(k_scatter, (unsigned)htiles.size(), tile, d_tiles.p, d_sys.p, src, rank.p, start.p,
            sorted.p, par.pair_kernel >= 2 ? fs.p : nullptr, counts.p, d_err.p);
   }
@@ -928,7 +928,7 @@ struct Engine {
 
   template <int MODE>
   void launch_pair() {
-    if (piles_up() && tile >= 128) chained = false;
+    if (pair_piles_up()) chained = false;
     const unsigned nt = (unsigned)htiles.size();
     if (par.pair_kernel == 4) {
       switch (typed_reaches<MODE>()) {
